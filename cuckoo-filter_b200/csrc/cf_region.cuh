@@ -337,14 +337,11 @@ __global__ void __launch_bounds__(kRgThreads) k_rg_probe(DevTable t, const uint6
         }
     }
     if constexpr (OP == SEG_INSERT) {
-        flush_counter(&t.ctr[round == 1 ? CTR_PRIMARY : CTR_SECONDARY], n_ok);
-        flush_counter(&t.ctr[CTR_OCCUPIED], n_ok);
+        flush_counters(t.ctr, {{round == 1 ? CTR_PRIMARY : CTR_SECONDARY, static_cast<int32_t>(n_ok)},
+                               {CTR_OCCUPIED, static_cast<int32_t>(n_ok)}});
     } else if constexpr (OP == SEG_DELETE) {
-        const uint32_t s = __reduce_add_sync(0xFFFFFFFFu, n_ok);
-        if (lane == 0 && s) {
-            atomicAdd(&t.ctr[CTR_REMOVED], static_cast<unsigned long long>(s));
-            atomicAdd(&t.ctr[CTR_OCCUPIED], ~static_cast<unsigned long long>(s) + 1ull);
-        }
+        const int32_t rem = static_cast<int32_t>(n_ok);
+        flush_counters(t.ctr, {{CTR_REMOVED, rem}, {CTR_OCCUPIED, -rem}});
     }
     if (__any_sync(0xFFFFFFFFu, err) && lane == 0) atomicOr(&t.ctr[CTR_ERROR], ERR_CAS_LIMIT);
 }

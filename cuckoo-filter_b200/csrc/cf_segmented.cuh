@@ -653,14 +653,11 @@ __global__ void __launch_bounds__(kSegThreads) k_seg(DevTable t, const uint64_t*
         __syncthreads();
     }
     if constexpr (OP == SEG_INSERT) {
-        flush_counter(&t.ctr[round == 2 ? CTR_SECONDARY : CTR_PRIMARY], n_ok);
-        flush_counter(&t.ctr[CTR_OCCUPIED], n_ok);
+        flush_counters(t.ctr, {{round == 2 ? CTR_SECONDARY : CTR_PRIMARY, static_cast<int32_t>(n_ok)},
+                               {CTR_OCCUPIED, static_cast<int32_t>(n_ok)}});
     } else if constexpr (OP == SEG_DELETE) {
-        const uint32_t s = __reduce_add_sync(0xFFFFFFFFu, n_ok);
-        if (lane == 0 && s) {
-            atomicAdd(&t.ctr[CTR_REMOVED], static_cast<unsigned long long>(s));
-            atomicAdd(&t.ctr[CTR_OCCUPIED], ~static_cast<unsigned long long>(s) + 1ull);
-        }
+        const int32_t rem = static_cast<int32_t>(n_ok);
+        flush_counters(t.ctr, {{CTR_REMOVED, rem}, {CTR_OCCUPIED, -rem}});
     }
     if (__any_sync(0xFFFFFFFFu, err) && lane == 0) atomicOr(&t.ctr[CTR_ERROR], ERR_CAS_LIMIT);
 }
@@ -863,10 +860,10 @@ __global__ void __launch_bounds__(256, C::nchunks <= 4 ? 3 : 2) k_evict_bfs_step
         if (outcome) has = false;
         if (err) has = false;  // a retry bound was hit: stop this key, the host reports the error
     }
-    flush_counter(&t.ctr[CTR_OCCUPIED], n_ok + n_dup);
-    flush_counter(&t.ctr[CTR_DUP], n_dup);
-    flush_counter(&t.ctr[CTR_EVICTED_INSERTS], count_keys ? n_evk : 0u);
-    flush_counter(&t.ctr[CTR_EVICTIONS], n_ev);
+    flush_counters(t.ctr, {{CTR_OCCUPIED, static_cast<int32_t>(n_ok + n_dup)},
+                           {CTR_DUP, static_cast<int32_t>(n_dup)},
+                           {CTR_EVICTED_INSERTS, static_cast<int32_t>(count_keys ? n_evk : 0u)},
+                           {CTR_EVICTIONS, static_cast<int32_t>(n_ev)}});
     if (__any_sync(0xFFFFFFFFu, err) && lane == 0) atomicOr(&t.ctr[CTR_ERROR], ERR_CAS_LIMIT);
 }
 
@@ -902,7 +899,7 @@ __device__ __forceinline__ uint32_t empty_count(const uint64_t (&c)[C::nchunks])
 // or whose compare-and-swap found a bucket changed, goes to `rest`, where the
 // step-machine BFS starts it over.  One key alone takes the reference's steps.
 template <class C, int P>
-__global__ void __launch_bounds__(256) k_evict_bfs_fast(DevTable t, const uint64_t* ent, const uint32_t* pay,
+__global__ void __launch_bounds__(256, C::nchunks <= 4 ? 3 : 2) k_evict_bfs_fast(DevTable t, const uint64_t* ent, const uint32_t* pay,
                                                         const unsigned long long* n_dev, uint32_t* bitmap,
                                                         uint64_t* rest, uint32_t* rest_pay,
                                                         unsigned long long* rest_count, uint32_t* full,
@@ -1015,10 +1012,10 @@ __global__ void __launch_bounds__(256) k_evict_bfs_fast(DevTable t, const uint64
             }
         }
     }
-    flush_counter(&t.ctr[CTR_OCCUPIED], n_ok + n_dup);
-    flush_counter(&t.ctr[CTR_DUP], n_dup);
-    flush_counter(&t.ctr[CTR_EVICTED_INSERTS], n_evk);
-    flush_counter(&t.ctr[CTR_EVICTIONS], n_ev);
+    flush_counters(t.ctr, {{CTR_OCCUPIED, static_cast<int32_t>(n_ok + n_dup)},
+                           {CTR_DUP, static_cast<int32_t>(n_dup)},
+                           {CTR_EVICTED_INSERTS, static_cast<int32_t>(n_evk)},
+                           {CTR_EVICTIONS, static_cast<int32_t>(n_ev)}});
     if (__any_sync(0xFFFFFFFFu, err) && lane == 0) atomicOr(&t.ctr[CTR_ERROR], ERR_CAS_LIMIT);
 }
 
@@ -1056,12 +1053,12 @@ __global__ void __launch_bounds__(256) k_evict_list(DevTable t, const uint64_t* 
             ++n_fail;
         }
     }
-    flush_counter(&t.ctr[CTR_OCCUPIED], n_evk - n_fail - st.lost + st.dup);
-    flush_counter(&t.ctr[CTR_DUP], st.dup);
-    flush_counter(&t.ctr[CTR_EVICTED_INSERTS], continued ? 0u : n_evk);
-    flush_counter(&t.ctr[CTR_EVICTIONS], st.evictions);
-    flush_counter(&t.ctr[CTR_FAILED], n_fail);
-    flush_counter(&t.ctr[CTR_LOST], st.lost);
+    flush_counters(t.ctr, {{CTR_OCCUPIED, static_cast<int32_t>(n_evk - n_fail - st.lost + st.dup)},
+                           {CTR_DUP, static_cast<int32_t>(st.dup)},
+                           {CTR_EVICTED_INSERTS, static_cast<int32_t>(continued ? 0u : n_evk)},
+                           {CTR_EVICTIONS, static_cast<int32_t>(st.evictions)},
+                           {CTR_FAILED, static_cast<int32_t>(n_fail)},
+                           {CTR_LOST, static_cast<int32_t>(st.lost)}});
     if (__any_sync(0xFFFFFFFFu, err) && (threadIdx.x & 31) == 0) atomicOr(&t.ctr[CTR_ERROR], ERR_CAS_LIMIT);
 }
 
@@ -1400,8 +1397,8 @@ __global__ void __launch_bounds__(kSegInsertThreads, 3) k_seg_insert(DevTable t,
         __syncthreads();
     }
     if (tid == 0) bulk_wait_all();
-    flush_counter(&t.ctr[round == 2 ? CTR_SECONDARY : CTR_PRIMARY], n_ok);
-    flush_counter(&t.ctr[CTR_OCCUPIED], n_ok);
+    flush_counters(t.ctr, {{round == 2 ? CTR_SECONDARY : CTR_PRIMARY, static_cast<int32_t>(n_ok)},
+                           {CTR_OCCUPIED, static_cast<int32_t>(n_ok)}});
 }
 
 // Round 2 by random access (few keys missed their primary bucket): entries
@@ -1452,19 +1449,16 @@ __global__ void __launch_bounds__(256) k_list_random(DevTable t, const uint64_t*
         }
     }
     if constexpr (OP == SEG_INSERT) {
-        flush_counter(&t.ctr[CTR_OCCUPIED], n_sec + n_evk - n_fail - st.lost + st.dup);
-        flush_counter(&t.ctr[CTR_DUP], st.dup);
-        flush_counter(&t.ctr[CTR_SECONDARY], n_sec);
-        flush_counter(&t.ctr[CTR_EVICTED_INSERTS], n_evk);
-        flush_counter(&t.ctr[CTR_EVICTIONS], st.evictions);
-        flush_counter(&t.ctr[CTR_FAILED], n_fail);
-        flush_counter(&t.ctr[CTR_LOST], st.lost);
+        flush_counters(t.ctr, {{CTR_OCCUPIED, static_cast<int32_t>(n_sec + n_evk - n_fail - st.lost + st.dup)},
+                               {CTR_DUP, static_cast<int32_t>(st.dup)},
+                               {CTR_SECONDARY, static_cast<int32_t>(n_sec)},
+                               {CTR_EVICTED_INSERTS, static_cast<int32_t>(n_evk)},
+                               {CTR_EVICTIONS, static_cast<int32_t>(st.evictions)},
+                               {CTR_FAILED, static_cast<int32_t>(n_fail)},
+                               {CTR_LOST, static_cast<int32_t>(st.lost)}});
     } else if constexpr (OP == SEG_DELETE) {
-        const uint32_t s = __reduce_add_sync(0xFFFFFFFFu, n_sec);
-        if ((threadIdx.x & 31) == 0 && s) {
-            atomicAdd(&t.ctr[CTR_REMOVED], static_cast<unsigned long long>(s));
-            atomicAdd(&t.ctr[CTR_OCCUPIED], ~static_cast<unsigned long long>(s) + 1ull);
-        }
+        const int32_t rem = static_cast<int32_t>(n_sec);
+        flush_counters(t.ctr, {{CTR_REMOVED, rem}, {CTR_OCCUPIED, -rem}});
     }
     if (__any_sync(0xFFFFFFFFu, err) && (threadIdx.x & 31) == 0) atomicOr(&t.ctr[CTR_ERROR], ERR_CAS_LIMIT);
 }
