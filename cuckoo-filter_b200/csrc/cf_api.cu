@@ -371,10 +371,13 @@ uint64_t auto_threshold(const cf_filter* f, int op) {
 // Batch size from which a batch is segment-staged.  Inserts: one key per
 // bucket (on B200 the segment path overtook random inserts between 0.5 and 1
 // key per bucket: 0.70 against 0.88 ms at 1, 0.98 against 1.73 ms at 2, on an
-// empty 2^28-slot table); lookups and deletes: eight keys per bucket.
+// empty 2^28-slot table); deletes: eight keys per bucket.  Lookups: never.
+// Random lookups were faster for every table and batch measured (256 KiB to
+// 2 GiB, 2 to 64 keys per bucket, random against segment-staged G/s: 97 and 21
+// in 8 MiB, 65 and 25 in 128 MiB, 36 and 24 in 512 MiB, 31.4 and 21.7 in 2 GiB).
 uint64_t segmented_threshold(const cf_filter* f, int op) {
     if (f->seg_min_keys) return f->seg_min_keys;
-    return op == SEG_INSERT ? f->num_buckets : f->num_buckets * 8;
+    return op == SEG_INSERT ? f->num_buckets : op == SEG_DELETE ? f->num_buckets * 8 : UINT64_MAX;
 }
 
 int run_segmented(cf_filter* f, int op, const void* keys, uint64_t n, uint8_t* out, void* stream) {

@@ -275,13 +275,37 @@ __device__ bool try_remove(uint64_t* bw, uint64_t (&c)[C::nchunks], uint32_t fp,
     return false;
 }
 
+// Does bucket image c hold tag fp?  Lookups in an L2-resident table are bound by
+// instruction issue, so the test is written for each tag width: 16-bit lanes
+// are folded with the three-input 16x2 minimum (a lane of the fold is 0 exactly
+// when some slot equals fp) and tested for a zero lane once per bucket, 32-bit
+// lanes are compared one by one, 8-bit lanes are tested for a zero lane word by
+// word (the borrow form: exact as a yes/no answer).
 template <class C>
 __device__ __forceinline__ bool has_tag(const uint64_t (&c)[C::nchunks], uint32_t fp) {
-    const uint64_t rep = replicate<C::bits>(fp);
-    uint64_t any = 0;
+    if constexpr (C::bits == 32) {
+        bool any = false;
 #pragma unroll
-    for (int j = 0; j < C::nchunks; ++j) any |= zero_lanes<C::bits>(c[j] ^ rep);
-    return any != 0;
+        for (int j = 0; j < C::nchunks; ++j)
+            any = any || static_cast<uint32_t>(c[j]) == fp || static_cast<uint32_t>(c[j] >> 32) == fp;
+        return any;
+    } else if constexpr (C::bits == 16) {
+        const uint32_t rep = fp * 0x00010001u;
+        uint32_t m = 0xFFFFFFFFu;
+#pragma unroll
+        for (int j = 0; j < C::nchunks; ++j)
+            m = __vimin3_u16x2(m, static_cast<uint32_t>(c[j]) ^ rep, static_cast<uint32_t>(c[j] >> 32) ^ rep);
+        return ((m - 0x00010001u) & ~m & 0x80008000u) != 0;
+    } else {
+        const uint32_t rep = fp * 0x01010101u;
+        uint32_t any = 0;
+#pragma unroll
+        for (int j = 0; j < C::nchunks; ++j) {
+            const uint32_t a = static_cast<uint32_t>(c[j]) ^ rep, b = static_cast<uint32_t>(c[j] >> 32) ^ rep;
+            any |= ((a - 0x01010101u) & ~a) | ((b - 0x01010101u) & ~b);
+        }
+        return (any & 0x80808080u) != 0;
+    }
 }
 
 // Atomically replace the tag in `slot`; returns the tag that was there.

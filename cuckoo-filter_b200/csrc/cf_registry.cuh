@@ -76,8 +76,13 @@ constexpr int kEvictGridWaves = 4;
 // segment-staged insert leaves free for the second round.
 constexpr uint32_t kRound1SlackSixteenths = 3;
 
-// Keys per thread of each batch kernel.
-constexpr int kContainsKPT = 4;
+// Keys per thread of each batch kernel.  Lookups: with 2 a thread needs 40
+// registers against 64 with 4, and the warps that fit beside it hide more
+// latency than the loads it gives up (20 M lookups, G/s at 4 -> 2 per thread:
+// 16-bit tags 122.9 -> 131.3 in an 8 MiB table, 59.0 -> 66.2 in 128 MiB; 8-bit
+// tags 45.4 -> 130.4 in 64 MiB, 32.6 -> 41.9 in 256 MiB; from 512 MiB on
+// within 2 %).
+constexpr int kContainsKPT = 2;
 constexpr int kDeleteKPT = 4;
 constexpr int kInsertKPT = 2;
 
@@ -175,7 +180,8 @@ struct Launchers {
     using Key = typename C::Key;
     // keys per thread; buckets wider than 64 bytes keep fewer in flight so
     // their images stay in registers
-    static constexpr int CKPT = C::bucket_bytes > 128 ? 1 : C::bucket_bytes > 64 ? 2 : kContainsKPT;
+    static constexpr int CKPT = C::bucket_bytes > 128 ? 1 : kContainsKPT;
+    static constexpr int KPT4 = C::bucket_bytes > 128 ? 1 : C::bucket_bytes > 64 ? 2 : 4;  // asked for 4
     static constexpr int DKPT = C::bucket_bytes > 64 ? 1 : kDeleteKPT;
     static constexpr int IKPT = C::bucket_bytes > 64 ? 1 : kInsertKPT;
 
@@ -231,6 +237,7 @@ struct Launchers {
         switch (L.kpt) {
             case 1: return contains_k<1>(t, keys, n, out, L);
             case 2: return contains_k<2>(t, keys, n, out, L);
+            case 4: return contains_k<KPT4>(t, keys, n, out, L);
             default: return contains_k<CKPT>(t, keys, n, out, L);
         }
     }
