@@ -146,11 +146,11 @@ __host__ __device__ __forceinline__ void candidates(uint64_t key, uint64_t nbm, 
     if constexpr (C::alt_policy == ALT_OFFSET) {
         // (bitsPerTag - 1) fingerprint bits, choice bit 0 (:232-247)
         const uint32_t f = static_cast<uint32_t>(h >> 32) & (C::choice_bit - 1u);
-        fp = f == 0 ? 1u : f;
+        fp = f > 1u ? f : 1u;  // 0 -> 1, as a maximum
         i1 = static_cast<uint64_t>(hb) % (nbm + 1);
     } else {
         const uint32_t f = static_cast<uint32_t>(h >> 32) & C::tag_mask;
-        fp = f == 0 ? 1u : f;
+        fp = f > 1u ? f : 1u;
         if constexpr (C::alt_policy == ALT_ADDSUB)
             i1 = static_cast<uint64_t>(hb) % ((nbm + 1) / 2);  // first half (:128-137)
         else

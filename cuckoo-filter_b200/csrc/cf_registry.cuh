@@ -12,6 +12,7 @@
 #include <cstdint>
 #include <vector>
 
+#include "cf_binned.cuh"
 #include "cf_kernels.cuh"
 #include "cf_region.cuh"
 #include "cf_segmented.cuh"
@@ -111,6 +112,10 @@ struct OpsTable {
     cudaError_t (*occupancy)(int kid, int block, int* blocks_per_sm);
     cudaError_t (*seg_chunk)(const DevTable&, const SegGeom&, const SegWork&, int op, const void* keys, uint64_t m,
                              uint8_t* out, cudaStream_t, uint32_t policy_bfs, uint32_t max_ev);
+    // binned insert of a whole batch, null where the configuration has none;
+    // *skewed: the batch does not hash evenly enough, and nothing has been stored
+    cudaError_t (*bin_insert)(const DevTable&, const BinGeom&, const BinWork&, const void* keys, uint64_t m, uint8_t* out,
+                              cudaStream_t, uint32_t policy_bfs, uint32_t max_ev, bool* skewed);
     cudaError_t (*rg_chunk)(const DevTable&, const RegionGeom&, const SegWork&, int op, const void* keys, uint64_t m,
                             uint8_t* out, cudaStream_t, uint32_t policy_bfs, uint32_t max_ev);
 };
@@ -445,6 +450,181 @@ struct Launchers {
         return cudaGetLastError();
     }
 
+    // Eviction of a list of keys whose buckets were full; `rest` is a second
+    // buffer of the list's size, and the list starts at entry *first (0 when null).  BFS: a lockstep pass over the first candidates,
+    // then the step machine for what it could not place, then DFS.
+    static void evict_left(const DevTable& t, uint64_t* list, uint32_t* list_pay, const unsigned long long* count,
+                           uint64_t* rest, uint32_t* rest_pay, unsigned long long* rest_count,
+                           unsigned long long* dfs_count, uint32_t* bitmap, uint8_t* fail_out, uint32_t* full, int sms,
+                           cudaStream_t s, uint32_t policy_bfs, uint32_t max_ev,
+                           const unsigned long long* first = nullptr) {
+        static const int list_bps = blocks_per_sm(k_evict_list<C>, 256, 0);
+        if (!policy_bfs) {
+            { k_evict_list<C><<<sms * list_bps * kEvictGridWaves, 256, 0, s>>>(t, list, list_pay, count, 0u, max_ev, bitmap,
+                                                                              0u, fail_out, first); CF_COUNT_LAUNCH(); }
+            return;
+        }
+        static const int fast_bps = blocks_per_sm(k_evict_bfs_fast<C, kBfsFastProbes>, 256, 0);
+        static const int bfs_bps = blocks_per_sm(k_evict_bfs_steps<C>, 256, 0);
+        // keys whose candidates all fail are flagged for DFS when entries leave bit 63 free
+        const int bucket_bits = t.nb_mask ? 64 - __builtin_clzll(t.nb_mask) : 0;
+        const uint32_t flag_ok = bucket_bits + C::bits <= 63 ? 1u : 0u;
+        { k_evict_bfs_fast<C, kBfsFastProbes><<<sms * fast_bps * kEvictGridWaves, 256, 0, s>>>(
+              t, list, list_pay, count, bitmap, rest, rest_pay, rest_count, full, flag_ok, first); CF_COUNT_LAUNCH(); }
+        { k_evict_bfs_steps<C><<<sms * bfs_bps * kEvictGridWaves, 256, 0, s>>>(t, rest, rest_pay, rest_count, bitmap, list,
+                                                                              list_pay, dfs_count, 0u); CF_COUNT_LAUNCH(); }
+        { k_evict_list<C><<<sms * list_bps * kEvictGridWaves, 256, 0, s>>>(t, list, list_pay, dfs_count, 0u, max_ev, bitmap,
+                                                                          1u, fail_out, nullptr); CF_COUNT_LAUNCH(); }
+    }
+
+    // One binning pass (see k_bin).  The tile is bin_ipt entries per thread, or 4 when
+    // that leaves SMs without one (small batches).
+    template <int SRC, typename EI, typename EO, bool PAY, int IPT>
+    static cudaError_t bin_pass_t(const BinArgs<EO>& a, int sms, uint64_t most, cudaStream_t s) {
+        constexpr auto kern = k_bin<C, SRC, EI, EO, PAY, IPT>;
+        constexpr size_t kMax = bin_smem<C, SRC, EI, PAY, IPT>(kBinMaxDigits);
+        cudaError_t e = ensure_smem_attr<kern>(static_cast<int>(kMax));
+        if (e != cudaSuccess) return e;
+        static const int bps = blocks_per_sm(kern, kBinThreads, kMax);
+        const uint64_t wave = static_cast<uint64_t>(sms) * bps;
+        const int grid = static_cast<int>(most < wave ? most : wave);
+        { kern<<<grid, kBinThreads, bin_smem<C, SRC, EI, PAY, IPT>(a.digits), s>>>(a); CF_COUNT_LAUNCH(); }
+        return cudaGetLastError();
+    }
+    template <int SRC, typename EI, typename EO, bool PAY>
+    static cudaError_t bin_pass(const BinArgs<EO>& a, int sms, uint64_t items, cudaStream_t s) {
+        constexpr int BIG = bin_ipt<PAY>(), SMALL = 4;
+        const bool big = items >= static_cast<uint64_t>(sms) * 2 * kBinThreads * BIG;
+        const uint64_t tile = static_cast<uint64_t>(kBinThreads) * (big ? BIG : SMALL);
+        const uint64_t most = SRC == BIN_KEYS    ? (items + tile - 1) / tile
+                              : SRC == BIN_SPLIT ? a.src_bins * ((a.src_cap + tile - 1) / tile)
+                                                 : a.src_bins;
+        return big ? bin_pass_t<SRC, EI, EO, PAY, BIG>(a, sms, most, s) : bin_pass_t<SRC, EI, EO, PAY, SMALL>(a, sms, most, s);
+    }
+    // The first pass of a round: the keys, or what the last round left in its segments' bins.
+    template <typename E2, typename EO, bool PAY>
+    static cudaError_t bin_first(BinArgs<EO> a, const void* keys, int sms, uint64_t items, cudaStream_t s) {
+        if (!keys) return bin_pass<BIN_LEFT, E2, EO, PAY>(a, sms, items, s);
+        a.src = keys;
+        return bin_pass<BIN_KEYS, uint32_t, EO, PAY>(a, sms, items, s);
+    }
+
+    // A whole batch through the binned path (cf_binned.cuh).
+    // E1: entries between the two passes; E2: entries of the segments' bins.
+    template <typename E1, typename E2, bool PAY>
+    static cudaError_t bin_insert_t(const DevTable& t, const BinGeom& g, const BinWork& w, const void* keys, uint64_t m,
+                                    uint8_t* out, cudaStream_t s, uint32_t policy_bfs, uint32_t max_ev, bool* skewed) {
+        const uint32_t cap1 = w.round1_cap ? w.round1_cap : m >= t.nb_mask + 1 ? round1_cap() : C::bs;
+        const int rounds = cap1 < static_cast<uint32_t>(C::bs) ? 3 : 2;
+        const uint32_t per_round = ((g.l2 ? g.d1 : 0u) + g.nseg) * kCursorStride;
+        cudaError_t e = cudaMemsetAsync(w.cnt, 0, 8 * sizeof(unsigned long long), s);
+        if (e == cudaSuccess) e = cudaMemsetAsync(w.cursor, 0, sizeof(uint32_t) * per_round * rounds, s);
+        if (e == cudaSuccess && w.full) e = cudaMemsetAsync(w.full, 0, w.full_words * sizeof(uint32_t), s);
+        if (e == cudaSuccess && PAY) e = cudaMemsetAsync(out, 1, m, s);  // failed keys are cleared at the end
+        const int smem = static_cast<int>((static_cast<size_t>(C::bucket_bytes) + 4) << g.sbl);
+        constexpr int kMaxSmem = kSegBytes + kSegBytes / C::bucket_bytes * 4;
+        if (e == cudaSuccess) e = ensure_smem_attr<k_bin_insert<C, E2, PAY, true>>(kMaxSmem);
+        if (e == cudaSuccess) e = ensure_smem_attr<k_bin_insert<C, E2, PAY, false>>(kMaxSmem);
+        int at = 0;  // the buffer of the segments' bins
+        for (int r = 1; r <= rounds && e == cudaSuccess; ++r) {
+            uint32_t* cur = w.cursor + static_cast<size_t>(per_round) * (r - 1);
+            uint32_t* seg_count = cur + (g.l2 ? g.d1 * kCursorStride : 0u);
+            const uint64_t items = r == 1 ? m : m / 4;  // an estimate after the first round
+            const int to = r == 1 ? 0 : 1 - at;
+            auto args = [&](auto* dst, bool first) {
+                BinArgs<typename std::remove_pointer<decltype(dst)>::type> a{};
+                a.n = m;
+                a.nb_mask = t.nb_mask;
+                a.dst = dst;
+                a.over = w.list;
+                a.over_pay = w.list_pay;
+                a.over_count = &w.cnt[0];
+                a.over_room = w.list_room;
+                a.out = out;
+                a.ctr = r == 1 ? nullptr : t.ctr;
+                a.over_alt = r != 2;
+                if (first) {
+                    a.src = w.ent[at];
+                    a.src_pay = w.pay[at];
+                    a.src_count = w.left;
+                    a.src_cap = g.room2;
+                    a.src_bins = g.nseg;
+                    a.left_sbl = g.sbl;
+                    a.low = g.sbl + g.l2;
+                    a.digits = g.d1;
+                    a.dst_pay = w.pay[to];
+                    a.cursor = cur;
+                    a.dst_cap = g.l2 ? g.room1 : g.room2;
+                } else {
+                    a.src = w.ent[to];
+                    a.src_pay = w.pay[to];
+                    a.src_count = cur;
+                    a.src_cap = g.room1;
+                    a.src_bins = g.d1;
+                    a.low = g.sbl;
+                    a.digits = 1u << g.l2;
+                    a.dst_pay = w.pay[1 - to];
+                    a.cursor = seg_count;
+                    a.dst_cap = g.room2;
+                }
+                return a;
+            };
+            const void* from = r == 1 ? keys : nullptr;
+            if (!g.l2) {
+                e = bin_first<E2, E2, PAY>(args(static_cast<E2*>(w.ent[to]), true), from, w.sms, items, s);
+                at = to;
+            } else {
+                e = bin_first<E2, E1, PAY>(args(static_cast<E1*>(w.ent[to]), true), from, w.sms, items, s);
+                if (e == cudaSuccess)
+                    e = bin_pass<BIN_SPLIT, E1, E2, PAY>(args(static_cast<E2*>(w.ent[1 - to]), false), w.sms, items, s);
+                at = 1 - to;
+            }
+            if (e != cudaSuccess) break;
+            if (r == 1 && w.list_room < m) {
+                // the list is shorter than the batch: a batch too skewed for it
+                // is left to the segment-staged path (nothing is stored yet)
+                e = cudaMemcpyAsync(w.h_cnt, &w.cnt[0], sizeof(unsigned long long), cudaMemcpyDeviceToHost, s);
+                if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+                if (e != cudaSuccess) break;
+                *skewed = w.h_cnt[0] > w.list_room;
+                if (*skewed) return cudaSuccess;
+            }
+            E2* ent = static_cast<E2*>(w.ent[at]);
+            const uint32_t cap = r == 1 ? cap1 : static_cast<uint32_t>(C::bs);
+            const int last = r == rounds;
+            if (r == 1 && w.fresh)
+                { k_bin_insert<C, E2, PAY, true><<<g.nseg, kBinInsertThreads, smem, s>>>(
+                      t, ent, w.pay[at], seg_count, g.room2, g.nseg, g.sbl, r, w.left, cap, last, w.list, w.list_pay,
+                      &w.cnt[3], &w.cnt[0], w.full); CF_COUNT_LAUNCH(); }
+            else
+                { k_bin_insert<C, E2, PAY, false><<<g.nseg, kBinInsertThreads, smem, s>>>(
+                      t, ent, w.pay[at], seg_count, g.room2, g.nseg, g.sbl, r, w.left, cap, last, w.list, w.list_pay,
+                      &w.cnt[3], &w.cnt[0], w.full); CF_COUNT_LAUNCH(); }
+            e = cudaGetLastError();
+        }
+        if (e != cudaSuccess) return e;
+        { k_bin_over<C><<<w.sms * 2, 256, 0, s>>>(t, w.list, w.list_pay, &w.cnt[0], policy_bfs, max_ev,
+                                                 PAY ? out : nullptr); CF_COUNT_LAUNCH(); }
+        evict_left(t, w.list, w.list_pay, &w.cnt[3], w.list + m, PAY ? w.list_pay + m : nullptr, &w.cnt[1], &w.cnt[2],
+                   nullptr, PAY ? out : nullptr, w.full, w.sms, s, policy_bfs, max_ev, &w.cnt[0]);
+        return cudaGetLastError();
+    }
+    static cudaError_t bin_insert(const DevTable& t, const BinGeom& g, const BinWork& w, const void* keys, uint64_t m,
+                                  uint8_t* out, cudaStream_t s, uint32_t policy_bfs, uint32_t max_ev, bool* skewed) {
+        if constexpr (C::bs > 16) {
+            return cudaErrorInvalidValue;
+        } else {
+            auto go = [&](auto e1, auto e2) {
+                return out ? bin_insert_t<decltype(e1), decltype(e2), true>(t, g, w, keys, m, out, s, policy_bfs, max_ev, skewed)
+                           : bin_insert_t<decltype(e1), decltype(e2), false>(t, g, w, keys, m, out, s, policy_bfs, max_ev, skewed);
+            };
+            if constexpr (C::bits < 32) {
+                if (g.entry_bytes2 == 4) return g.entry_bytes1 == 4 ? go(uint32_t{}, uint32_t{}) : go(uint64_t{}, uint32_t{});
+            }
+            return go(uint64_t{}, uint64_t{});
+        }
+    }
+
     template <int OP>
     static cudaError_t seg_chunk_op(const DevTable& t, const SegGeom& g, const SegWork& w, const void* keys,
                                     uint64_t m, uint8_t* out, cudaStream_t s, uint32_t policy_bfs, uint32_t max_ev) {
@@ -504,31 +684,9 @@ struct Launchers {
                     }
                 }
                 if (e == cudaSuccess && OP == SEG_INSERT && evict) {
-                    uint32_t* bm = payload ? w.bitmap : nullptr;
-                    static const int bfs_bps = blocks_per_sm(k_evict_bfs_steps<C>, 256, 0);
-                    static const int list_bps = blocks_per_sm(k_evict_list<C>, 256, 0);
-                    if (policy_bfs) {
-                        // a lockstep pass over the first candidates, then the
-                        // step machine for what it could not place, then DFS
-                        static const int fast_bps = blocks_per_sm(k_evict_bfs_fast<C, kBfsFastProbes>, 256, 0);
-                        uint32_t* p_in = payload ? w.pay[1 - c] : nullptr;
-                        uint32_t* p_mid = payload ? w.pay[c] : nullptr;
-                        // keys whose candidates all fail are flagged for DFS when
-                        // entries leave bit 63 free
-                        const int bucket_bits = t.nb_mask ? 64 - __builtin_clzll(t.nb_mask) : 0;
-                        const uint32_t flag_ok = bucket_bits + C::bits <= 63 ? 1u : 0u;
-                        { k_evict_bfs_fast<C, kBfsFastProbes><<<w.sms * fast_bps * kEvictGridWaves, 256, 0, s>>>(
-                              t, w.ent[1 - c], p_in, left, bm, w.ent[c], p_mid, &w.cnt[4], w.full, flag_ok);
-                          CF_COUNT_LAUNCH(); }
-                        { k_evict_bfs_steps<C><<<w.sms * bfs_bps * kEvictGridWaves, 256, 0, s>>>(
-                              t, w.ent[c], p_mid, &w.cnt[4], bm, w.ent[1 - c], p_in, &w.cnt[2], 0u); CF_COUNT_LAUNCH(); }
-                        { k_evict_list<C><<<w.sms * list_bps * kEvictGridWaves, 256, 0, s>>>(t, w.ent[1 - c], p_in,
-                                                                        &w.cnt[2], 0u, max_ev, bm, 1u); CF_COUNT_LAUNCH(); }
-                    } else {
-                        { k_evict_list<C><<<w.sms * list_bps * kEvictGridWaves, 256, 0, s>>>(t, w.ent[1 - c],
-                                                                        payload ? w.pay[1 - c] : nullptr, left,
-                                                                        0u, max_ev, bm, 0u); CF_COUNT_LAUNCH(); }
-                    }
+                    evict_left(t, w.ent[1 - c], payload ? w.pay[1 - c] : nullptr, left, w.ent[c],
+                               payload ? w.pay[c] : nullptr, &w.cnt[4], &w.cnt[2], payload ? w.bitmap : nullptr, nullptr,
+                               w.full, w.sms, s, policy_bfs, max_ev);
                 }
             } else {
                 const int lgrid = static_cast<int>((m2 + 255) / 256 < 8192 ? (m2 + 255) / 256 : 8192);
@@ -622,9 +780,9 @@ struct Launchers {
                 if (policy_bfs) {
                     { k_evict_bfs_steps<C><<<w.sms * bfs_bps * kEvictGridWaves, 256, 0, s>>>(t, w.ent[1], p1, &w.cnt[1], bm, w.ent[0], p0,
                                                                        &w.cnt[2], 1u); CF_COUNT_LAUNCH(); }
-                    { k_evict_list<C><<<w.sms * list_bps * kEvictGridWaves, 256, 0, s>>>(t, w.ent[0], p0, &w.cnt[2], 0u, max_ev, bm, 1u); CF_COUNT_LAUNCH(); }
+                    { k_evict_list<C><<<w.sms * list_bps * kEvictGridWaves, 256, 0, s>>>(t, w.ent[0], p0, &w.cnt[2], 0u, max_ev, bm, 1u, nullptr, nullptr); CF_COUNT_LAUNCH(); }
                 } else {
-                    { k_evict_list<C><<<w.sms * list_bps * kEvictGridWaves, 256, 0, s>>>(t, w.ent[1], p1, &w.cnt[1], 0u, max_ev, bm, 0u); CF_COUNT_LAUNCH(); }
+                    { k_evict_list<C><<<w.sms * list_bps * kEvictGridWaves, 256, 0, s>>>(t, w.ent[1], p1, &w.cnt[1], 0u, max_ev, bm, 0u, nullptr, nullptr); CF_COUNT_LAUNCH(); }
                 }
             }
         }
@@ -665,6 +823,7 @@ struct Launchers {
         o.probe = probe;
         o.occupancy = occupancy;
         o.seg_chunk = seg_chunk;
+        o.bin_insert = C::bs <= 16 ? bin_insert : nullptr;
         o.rg_chunk = rg_chunk;
         return o;
     }

@@ -903,11 +903,15 @@ __global__ void __launch_bounds__(256, C::nchunks <= 4 ? 3 : 2) k_evict_bfs_fast
                                                         const unsigned long long* n_dev, uint32_t* bitmap,
                                                         uint64_t* rest, uint32_t* rest_pay,
                                                         unsigned long long* rest_count, uint32_t* full,
-                                                        uint32_t flag_ok) {
+                                                        uint32_t flag_ok, const unsigned long long* first_dev) {
     constexpr uint64_t lane_mask = C::bits == 32 ? 0xFFFFFFFFULL : ((1ULL << C::bits) - 1ULL);
     constexpr int NC = (C::bs / 2) < 8 ? (C::bs / 2) : 8;
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t lt_mask = (1u << lane) - 1u;
+    if (first_dev) {
+        ent += *first_dev;
+        if (pay) pay += *first_dev;
+    }
     const uint64_t m = *n_dev;
     uint32_t n_evk = 0, n_ok = 0, n_ev = 0, n_dup = 0;
     bool err = false;
@@ -1021,11 +1025,18 @@ __global__ void __launch_bounds__(256, C::nchunks <= 4 ? 3 : 2) k_evict_bfs_fast
 
 // Eviction for the keys whose two buckets were full after both segment rounds
 // (or, with `continued`, whose BFS candidates all failed); entries carry
-// (alternate bucket, tag).  One key per thread, all lanes busy.
+// (alternate bucket, tag).  One key per thread, all lanes busy.  Results: a
+// stored key's bit is set in `bitmap`, or a failed key's byte cleared in `fail_out`.
+// The list starts at entry *first_dev (0 when null).
 template <class C>
 __global__ void __launch_bounds__(256) k_evict_list(DevTable t, const uint64_t* ent, const uint32_t* pay,
                                                     const unsigned long long* n_dev, uint32_t policy_bfs,
-                                                    uint32_t max_ev, uint32_t* bitmap, uint32_t continued) {
+                                                    uint32_t max_ev, uint32_t* bitmap, uint32_t continued,
+                                                    uint8_t* fail_out, const unsigned long long* first_dev) {
+    if (first_dev) {
+        ent += *first_dev;
+        if (pay) pay += *first_dev;
+    }
     const uint64_t m = *n_dev;
     uint32_t n_evk = 0, n_fail = 0;
     EvictStats st;
@@ -1051,6 +1062,7 @@ __global__ void __launch_bounds__(256) k_evict_list(DevTable t, const uint64_t* 
             }
         } else {
             ++n_fail;
+            if (fail_out) fail_out[pay[i]] = 0;
         }
     }
     flush_counters(t.ctr, {{CTR_OCCUPIED, static_cast<int32_t>(n_evk - n_fail - st.lost + st.dup)},

@@ -47,3 +47,116 @@ def test_lookups_tell_near_misses_apart(cfb, orc, kb, bits, bs, per_bucket):
     f.setOption(cfb.OPT_STAGING, cfb.STAGING_SEGMENT)
     assert np.array_equal(host_u8(f.containsMany(d)), want)
     assert np.array_equal(image(f), o.table)
+
+
+POLICY = {"xor": "XorAltBucketPolicy", "addsub": "AddSubAltBucketPolicy", "offset": "OffsetAltBucketPolicy"}
+
+
+def filled_and_emptied(cfb, f, batches, results, sorted_=False):
+    """Inserts the batches, then checks the table by what it answers and by
+    taking every key out again: a wrong or missing entry leaves a delete that
+    fails or a slot that is not zero."""
+    total = 0
+    for keys in batches:
+        ok = torch.zeros(keys.numel(), dtype=torch.bool, device="cuda") if results else None
+        total += keys.numel()
+        occ = (f.insertManySorted if sorted_ else f.insertMany)(keys, d_output=ok)
+        assert occ == total == f.countOccupiedSlots()
+        assert ok is None or bool(ok.all())
+    st = f.stats()
+    assert st["failed"] == st["lost"] == st["duplicates"] == 0
+    assert st["primary"] + st["secondary"] + st["evicted_inserts"] == total
+    for keys in batches:
+        assert bool(f.containsMany(keys).all())
+    for keys in batches:
+        gone = torch.zeros(keys.numel(), dtype=torch.bool, device="cuda")
+        total -= keys.numel()
+        assert f.deleteMany(keys, gone) == total and bool(gone.all())
+    assert int(f.table_image().to(torch.int32).sum()) == 0
+
+
+@pytest.mark.parametrize("results", [False, True])
+@pytest.mark.parametrize("kb,bits,bs,alt,slots,loads", [
+    (8, 16, 16, "xor", 16, (0.5,)),                    # one bucket
+    (8, 16, 16, "xor", 1 << 8, (0.5, 0.3)),            # one segment
+    (8, 16, 16, "xor", 1 << 14, (0.0625, 0.7)),        # exactly one key per bucket
+    (4, 16, 16, "xor", 1 << 20, (0.5, 0.4)),           # one pass, a table that is not empty
+    (8, 8, 16, "xor", 1 << 20, (0.9,)),
+    (8, 8, 8, "xor", 1 << 18, (0.5, 0.3)),             # 8-byte buckets
+    (8, 16, 4, "xor", 1 << 18, (0.85,)),
+    (8, 32, 8, "xor", 1 << 19, (0.4, 0.45)),           # 8-byte entries
+    (4, 32, 2, "xor", 1 << 16, (0.55,)),
+    (8, 16, 16, "addsub", 1_000_003, (0.6, 0.3)),      # partial last segment, primary buckets in one half
+    (4, 16, 16, "offset", 777_777, (0.5, 0.4)),
+    (8, 16, 16, "offset", 100, (0.7,)),
+    (8, 16, 16, "xor", 1 << 25, (0.1, 0.2)),           # two passes, 4-byte entries between them
+    (8, 32, 8, "xor", 1 << 24, (0.3,)),                # two passes, 8-byte entries
+    (8, 16, 16, "offset", 20_000_000, (0.2,)),         # two passes, partial last segment
+])
+def test_binned_insert_stores_exactly_the_batch(cfb, orc, kb, bits, bs, alt, slots, loads, results):
+    policy = cfb.EvictionPolicy(int(results))
+    cfg = cfb.CuckooConfig(T="uint64" if kb == 8 else "uint32", bitsPerTag=bits, bucketSize=bs, maxEvictions=500,
+                           AltBucketPolicy=POLICY[alt], evictionPolicy=policy)
+    f = cfb.CuckooFilter(cfg, slots)
+    cap, batches, at = f.capacity(), [], 0
+    for load in loads:
+        n = max(f.getNumBuckets(), int(load * cap))
+        keys = orc.splitmix64(11 + bits + bs, n, first=at)
+        at += n
+        if kb == 4:
+            keys = keys.astype(np.uint32)
+        batches.append(dev(keys))
+    filled_and_emptied(cfb, f, batches, results, sorted_=bits == 32)
+    f.close()
+
+
+def test_binned_insert_with_entries_of_both_widths(cfb, orc):
+    """A 1 GiB table: 8-byte entries between the passes, 4-byte ones in the segments' bins."""
+    cfg = cfb.CuckooConfig(T="uint64", bitsPerTag=16, bucketSize=16, evictionPolicy=cfb.EvictionPolicy.BFS)
+    f = cfb.CuckooFilter(cfg, 1 << 29)
+    n = f.getNumBuckets()
+    filled_and_emptied(cfb, f, [dev(orc.splitmix64(5, n + 1)), dev(orc.splitmix64(5, n + 777, first=n + 1))], False)
+    f.close()
+
+
+@pytest.mark.parametrize("kb,bits,bs,slots,hot,copies,limit", [
+    (8, 16, 16, 1 << 16, 1, 5000, 0),       # one value repeated past its segment's bin
+    (8, 16, 16, 1 << 16, 40, 300, 0),
+    (8, 16, 16, 1 << 25, 3, 700_000, 0),    # past a first-pass bin and past a segment's bin
+    (8, 32, 8, 1 << 24, 1, 1_800_000, 0),
+    (8, 32, 8, 1 << 24, 1, 1_800_000, 80),  # a list of half the batch, too short: the segment-staged path
+    (8, 32, 8, 1 << 24, 1, 300_000, 80),    # a list of half the batch that suffices
+])
+@pytest.mark.parametrize("results", [False, True])
+def test_binned_insert_of_repeated_keys(cfb, orc, kb, bits, bs, slots, hot, copies, limit, results):
+    """Batches that do not hash evenly: what fits is stored, every other key of the
+    batch is, and the counters and flags agree with the table."""
+    if limit and results:
+        limit = 120
+    cfg = cfb.CuckooConfig(T="uint64", bitsPerTag=bits, bucketSize=bs, maxEvictions=4,
+                           evictionPolicy=cfb.EvictionPolicy.BFS)
+    f = cfb.CuckooFilter(cfg, slots)
+    if limit:
+        f.setOption(cfb.OPT_WORKSPACE_LIMIT, limit << 20)
+    rest = orc.splitmix64(21, max(f.getNumBuckets(), int(0.15 * slots)))
+    hots = orc.splitmix64(22, hot)
+    keys = np.concatenate([np.repeat(hots, copies), rest])
+    keys = keys[np.random.default_rng(4).permutation(len(keys))]
+    d = dev(keys)
+    ok = torch.zeros(len(keys), dtype=torch.bool, device="cuda") if results else None
+    occ = f.insertMany(d, d_output=ok)
+    st = f.stats()
+    assert occ == f.countOccupiedSlots() == len(keys) - st["failed"] - st["lost"] + st["duplicates"]
+    assert st["failed"] >= hot * (copies - 2 * bs) - st["lost"]
+    assert bool(f.containsMany(dev(hots)).all())
+    if results:
+        assert int(ok.sum()) == len(keys) - st["failed"]
+    if st["lost"] == 0:
+        # a key fails only when both its buckets are buckets of repeated values, which
+        # are full of them: any other key's second bucket has room at this load
+        c = cfb.CuckooFilter.getCandidateBuckets(cfg, rest, f.getNumBuckets())
+        h = cfb.CuckooFilter.getCandidateBuckets(cfg, hots, f.getNumBuckets())
+        full = np.unique(np.concatenate(h[:2]))
+        hopeless = np.isin(c[0], full) & np.isin(c[1], full)
+        assert np.all(host_u8(f.containsMany(dev(rest))).astype(bool) | hopeless)
+    f.close()
