@@ -4,15 +4,18 @@
 // of a persistent kernel.  The work list lives in device memory: item j is the
 // key range [offs[j], offs[j+1]) of the concatenated key buffer, destined for
 // filter filt[j] (offs is monotonic, offs[n_items] = total keys).  The grid
-// strides over tiles of the concatenated keys; each thread finds the item of
-// its first key by binary search over offs and walks forward from there, so
-// no per-item scratch or host-side tiling is needed and the launch can be
-// captured in a CUDA graph and replayed with new keys in the same buffers.
+// strides over tiles of the concatenated keys; a CTA finds the items of its
+// tile's first and last key by binary search over offs, and each thread searches
+// between those and walks forward, so no per-item scratch or host-side tiling
+// is needed and the launch can be captured in a CUDA graph and replayed with
+// new keys in the same buffers.
 //
 // Per-key semantics are the single-filter kernels' (cf_kernels.cuh): the
 // reference's insert / contains / remove (CuckooFilter.cuh:805-1116) applied
-// to the filter the key belongs to.  Counters are per filter; a warp adds its
-// lanes' counts with one atomic per distinct filter (__match_any_sync).
+// to the filter the key belongs to.  Counters are per filter; a warp whose keys
+// all belong to one filter (nearly every warp) adds each count with one
+// reduction and one atomic, any other with one atomic per distinct filter
+// (__match_any_sync).
 //
 // Tunables (template parameters, picked by the set's autotuner): KPT keys per
 // thread, and for lookups the probe width W: W lanes cooperate on one key,
@@ -25,9 +28,8 @@
 
 namespace cfb {
 
-// Item of key k: the largest j with offs[j] <= k (empty items are skipped).
-__device__ __forceinline__ uint32_t set_find_item(const uint64_t* __restrict__ offs, uint32_t n_items, uint64_t k) {
-    uint32_t lo = 0, hi = n_items;
+// Item of key k in [lo, hi): the largest j with offs[j] <= k (empty items are skipped).
+__device__ __forceinline__ uint32_t set_find_item(const uint64_t* __restrict__ offs, uint32_t lo, uint32_t hi, uint64_t k) {
     while (hi - lo > 1) {
         const uint32_t mid = (lo + hi) >> 1;
         if (offs[mid] <= k) lo = mid; else hi = mid;
@@ -35,12 +37,30 @@ __device__ __forceinline__ uint32_t set_find_item(const uint64_t* __restrict__ o
     return lo;
 }
 
-// Advance item j (an item of some key <= k) to the item of key k.
-__device__ __forceinline__ uint32_t set_advance(const uint64_t* __restrict__ offs, uint32_t n_items, uint32_t j,
-                                                uint64_t k) {
-    while (j + 1 < n_items && offs[j + 1] <= k) ++j;
-    return j;
+// Items of the tile [first, last]: range[0] of its first key, range[1] past that
+// of its last.  Every thread of the CTA calls it, between two barriers of its own.
+__device__ __forceinline__ void set_tile_items(const uint64_t* __restrict__ offs, uint32_t n_items, uint64_t first,
+                                               uint64_t last, uint32_t (&range)[2]) {
+    __syncthreads();
+    if (threadIdx.x == 0) range[0] = set_find_item(offs, 0, n_items, first);
+    if (threadIdx.x == 32 % blockDim.x) range[1] = set_find_item(offs, 0, n_items, last) + 1;
+    __syncthreads();
 }
+
+// A thread's walk over the items of its consecutive keys.
+struct SetWalk {
+    uint32_t item;
+    uint64_t end;  // first key past the item (and past the empty ones after it)
+    __device__ __forceinline__ SetWalk(const uint64_t* __restrict__ offs, const uint32_t (&range)[2], uint64_t k)
+        : item(set_find_item(offs, range[0], range[1], k)), end(offs[item + 1]) {}
+    // moves to the item of key k; true when that is another one
+    __device__ __forceinline__ bool to(const uint64_t* __restrict__ offs, uint32_t n_items, uint64_t k) {
+        if (k < end) return false;
+        while (item + 1 < n_items && offs[item + 1] <= k) ++item;
+        end = offs[item + 1];
+        return true;
+    }
+};
 
 constexpr uint64_t ERR_BAD_FILTER = 4;  // a work item named a filter outside the set
 
@@ -51,77 +71,106 @@ __device__ __forceinline__ uint32_t set_filter(const uint32_t* __restrict__ filt
     return f < n_filters ? f : n_filters;
 }
 
-// Adds v (per lane) to counter `idx` of filter f (per lane): one atomic per
-// distinct filter of the warp.  All lanes of the warp must call it.
-__device__ __forceinline__ void set_add_ctr(const DevTable* __restrict__ descs, uint32_t f, bool active, int idx,
-                                            uint32_t v) {
-    const uint32_t key = active ? f : 0xFFFFFFFFu;
-    const uint32_t peers = __match_any_sync(0xFFFFFFFFu, key);
-    uint32_t s = 0;
-    for (uint32_t m = peers; m; m &= m - 1) s += __shfl_sync(peers, v, __ffs(m) - 1);
-    const int lane = threadIdx.x & 31;
-    if (active && lane == __ffs(peers) - 1 && s) {
-        if (idx == CTR_REMOVED) {
-            atomicAdd(&descs[f].ctr[CTR_REMOVED], static_cast<unsigned long long>(s));
-            atomicAdd(&descs[f].ctr[CTR_OCCUPIED], ~static_cast<unsigned long long>(s) + 1ull);
+// Adds each lane's values to the counters of its filter f: one atomic per
+// counter when the active lanes share a filter, else one per distinct filter.
+// All lanes of the warp must call it.
+template <int N>
+__device__ __forceinline__ void set_add_ctrs(const DevTable* __restrict__ descs, uint32_t f, bool active,
+                                             const CounterAdd (&a)[N]) {
+    const uint32_t lane = threadIdx.x & 31, act = __ballot_sync(0xFFFFFFFFu, active);
+    if (!act) return;
+    const uint32_t f0 = __shfl_sync(0xFFFFFFFFu, f, __ffs(act) - 1);
+    uint32_t peers = act;
+    const bool one = __all_sync(0xFFFFFFFFu, !active || f == f0);
+    if (!one) peers = __match_any_sync(0xFFFFFFFFu, active ? f : 0xFFFFFFFFu);
+    const bool leader = active && lane == static_cast<uint32_t>(__ffs(peers) - 1);
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        int32_t s = 0;
+        if (one) {
+            s = __reduce_add_sync(0xFFFFFFFFu, active ? a[i].v : 0);
         } else {
-            atomicAdd(&descs[f].ctr[idx], static_cast<unsigned long long>(s));
+            for (uint32_t m = peers; m; m &= m - 1) s += __shfl_sync(peers, a[i].v, __ffs(m) - 1);
         }
+        if (leader && s) atomicAdd(&descs[f].ctr[a[i].idx], static_cast<unsigned long long>(static_cast<long long>(s)));
     }
 }
 
+// Keys of a thread that are probed together: their bucket loads overlap, and two
+// images leave registers for twice the warps that four would.
+template <int KPT>
+constexpr int set_batch() {
+    return KPT < 2 ? 1 : 2;
+}
+
 // containsMany over the set, W = 1: each thread owns KPT consecutive keys.
+// Bound by instruction issue: 512 filters of 1 K to 1 M slots, 14.2 M keys, took
+// 219 us with a binary search over all items per thread, four images per
+// thread and single-byte stores, and take 150.
 template <class C, int KPT>
 __global__ void __launch_bounds__(512) k_set_contains1(const DevTable* __restrict__ descs,
                                                        const uint32_t* __restrict__ filt,
                                                        const uint64_t* __restrict__ offs, uint32_t n_items, uint32_t n_filters,
                                                        const typename C::Key* __restrict__ keys, uint64_t n,
                                                        uint8_t* __restrict__ out, unsigned long long* err_flag) {
+    constexpr int B = set_batch<KPT>();
+    __shared__ uint32_t s_items[2];
     const uint64_t tile = static_cast<uint64_t>(blockDim.x) * KPT;
+    const bool keys_vec = reinterpret_cast<uintptr_t>(keys) % (KPT * C::key_bytes < 32 ? KPT * C::key_bytes : 32) == 0;
+    const bool out_vec = reinterpret_cast<uintptr_t>(out) % KPT == 0;
     bool bad = false;
     for (uint64_t base = blockIdx.x * tile; base < n; base += static_cast<uint64_t>(gridDim.x) * tile) {
+        set_tile_items(offs, n_items, base, (base + tile < n ? base + tile : n) - 1, s_items);
         const uint64_t k0 = base + static_cast<uint64_t>(threadIdx.x) * KPT;
         if (k0 >= n) continue;
-        uint32_t item = set_find_item(offs, n_items, k0);
-        uint32_t valid = 0;  // keys of this thread that exist and name a filter of the set
-        DevTable t[KPT];
-        uint64_t b[KPT];
-        uint32_t fp[KPT];
-        uint64_t c[KPT][C::nchunks];
+        uint64_t key[KPT];
+        load_keys<C, KPT>(keys, k0, n, keys_vec, key);
+        SetWalk walk(offs, s_items, k0);
+        uint32_t f = set_filter(filt, walk.item, n_filters);
+        DevTable cur = descs[f < n_filters ? f : 0];
+        uint32_t hit = 0;
 #pragma unroll
-        for (int j = 0; j < KPT; ++j) {
-            const uint64_t k = k0 + j;
-            if (k < n) {
-                item = set_advance(offs, n_items, item, k);
-                const uint32_t f = set_filter(filt, item, n_filters);
+        for (int g = 0; g < KPT; g += B) {
+            uint32_t live = 0;  // keys that exist and name a filter of the set
+            uint8_t* tb[B];
+            uint64_t mask[B], b[B];
+            uint32_t fp[B];
+            uint64_t c[B][C::nchunks];
+#pragma unroll
+            for (int j = 0; j < B; ++j) {
+                const uint64_t k = k0 + g + j;
+                if (k >= n) continue;
+                if (walk.to(offs, n_items, k)) {
+                    f = set_filter(filt, walk.item, n_filters);
+                    cur = descs[f < n_filters ? f : 0];
+                }
                 if (f == n_filters) {
                     bad = true;
                     continue;
                 }
-                valid |= 1u << j;
-                t[j] = descs[f];
-                candidates<C>(static_cast<uint64_t>(keys[k]), t[j].nb_mask, b[j], fp[j]);
-                load_nc<C::bucket_bytes>(t[j].buckets + b[j] * C::bucket_bytes, c[j]);
+                live |= 1u << j;
+                tb[j] = cur.buckets;
+                mask[j] = cur.nb_mask;
+                candidates<C>(key[g + j], mask[j], b[j], fp[j]);
+                load_nc<C::bucket_bytes>(tb[j] + b[j] * C::bucket_bytes, c[j]);
             }
-        }
-        uint32_t hit = 0;
+            uint32_t in = 0;
 #pragma unroll
-        for (int j = 0; j < KPT; ++j)
-            if (((valid >> j) & 1u) && has_tag<C>(c[j], fp[j])) hit |= 1u << j;
+            for (int j = 0; j < B; ++j)
+                if (((live >> j) & 1u) && has_tag<C>(c[j], fp[j])) in |= 1u << j;
 #pragma unroll
-        for (int j = 0; j < KPT; ++j) {
-            if (((valid >> j) & 1u) && !((hit >> j) & 1u)) {
-                b[j] = alt_bucket<C>(b[j], fp[j], t[j].nb_mask);
-                fp[j] = alt_tag<C>(fp[j]);  // the tag in the alternate bucket's form
-                load_nc<C::bucket_bytes>(t[j].buckets + b[j] * C::bucket_bytes, c[j]);
+            for (int j = 0; j < B; ++j) {
+                if (((live & ~in) >> j) & 1u) {
+                    b[j] = alt_bucket<C>(b[j], fp[j], mask[j]);
+                    load_nc<C::bucket_bytes>(tb[j] + b[j] * C::bucket_bytes, c[j]);
+                }
             }
-        }
 #pragma unroll
-        for (int j = 0; j < KPT; ++j) {
-            if (k0 + j >= n) break;
-            if (((valid >> j) & 1u) && !((hit >> j) & 1u) && has_tag<C>(c[j], fp[j])) hit |= 1u << j;
-            out[k0 + j] = static_cast<uint8_t>((hit >> j) & 1u);
+            for (int j = 0; j < B; ++j)
+                if ((((live & ~in) >> j) & 1u) && has_tag<C>(c[j], alt_tag<C>(fp[j]))) in |= 1u << j;
+            hit |= in << g;
         }
+        store_results<KPT>(out, k0, n, out_vec, hit);
     }
     if (bad) atomicOr(err_flag, ERR_BAD_FILTER);
 }
@@ -145,7 +194,7 @@ __global__ void __launch_bounds__(512) k_set_containsW(const DevTable* __restric
     const uint64_t tile = groups * KPT;
     for (uint64_t base = blockIdx.x * tile; base < n; base += static_cast<uint64_t>(gridDim.x) * tile) {
         const uint64_t k0 = base + static_cast<uint64_t>(threadIdx.x / W) * KPT;
-        uint32_t item = k0 < n ? set_find_item(offs, n_items, k0) : 0;
+        uint32_t item = k0 < n ? set_find_item(offs, 0, n_items, k0) : 0;
         DevTable t[KPT];
         uint64_t b[KPT];
         uint32_t fp[KPT];
@@ -157,7 +206,7 @@ __global__ void __launch_bounds__(512) k_set_containsW(const DevTable* __restric
             piece[j] = 0;
             fp[j] = 1;
             if (k < n) {
-                item = set_advance(offs, n_items, item, k);
+                while (item + 1 < n_items && offs[item + 1] <= k) ++item;
                 const uint32_t f = set_filter(filt, item, n_filters);
                 if (f == n_filters) {
                     bad = true;
@@ -193,51 +242,92 @@ __global__ void __launch_bounds__(512) k_set_containsW(const DevTable* __restric
     if (bad) atomicOr(err_flag, ERR_BAD_FILTER);
 }
 
-// deleteMany over the set: each thread owns KPT consecutive keys.
+// deleteMany over the set: each thread owns KPT consecutive keys.  The keys of
+// the thread's first filter are worked on together; those past the filter's end
+// (a few threads per item) follow one at a time, so the common path keeps one
+// table descriptor in registers.
 template <class C, int KPT>
-__global__ void __launch_bounds__(512) k_set_delete(const DevTable* __restrict__ descs, const uint32_t* __restrict__ filt,
-                                                    const uint64_t* __restrict__ offs, uint32_t n_items, uint32_t n_filters,
-                                                    const typename C::Key* __restrict__ keys, uint64_t n,
-                                                    uint8_t* __restrict__ out, unsigned long long* err_flag) {
+__global__ void __launch_bounds__(512, 2) k_set_delete(const DevTable* __restrict__ descs, const uint32_t* __restrict__ filt,
+                                                       const uint64_t* __restrict__ offs, uint32_t n_items,
+                                                       uint32_t n_filters, const typename C::Key* __restrict__ keys, uint64_t n,
+                                                       uint8_t* __restrict__ out, unsigned long long* err_flag) {
+    constexpr int B = set_batch<KPT>();
+    __shared__ uint32_t s_items[2];
     const uint64_t tile = static_cast<uint64_t>(blockDim.x) * KPT;
+    const bool keys_vec = reinterpret_cast<uintptr_t>(keys) % (KPT * C::key_bytes < 32 ? KPT * C::key_bytes : 32) == 0;
+    const bool out_vec = reinterpret_cast<uintptr_t>(out) % KPT == 0;
     bool err = false, bad = false;
     for (uint64_t base = blockIdx.x * tile; base < n; base += static_cast<uint64_t>(gridDim.x) * tile) {
+        set_tile_items(offs, n_items, base, (base + tile < n ? base + tile : n) - 1, s_items);
         const uint64_t k0 = base + static_cast<uint64_t>(threadIdx.x) * KPT;
-        uint32_t item = k0 < n ? set_find_item(offs, n_items, k0) : 0;
+        const uint32_t have = k0 < n ? (n - k0 < KPT ? static_cast<uint32_t>(n - k0) : KPT) : 0u;
+        uint64_t key[KPT];
+        if (have) load_keys<C, KPT>(keys, k0, n, keys_vec, key);
+        SetWalk walk(offs, s_items, have ? k0 : base);
+        uint32_t f = set_filter(filt, walk.item, n_filters);
+        bad |= have && f == n_filters;
+        const DevTable t = descs[f < n_filters ? f : 0];
+        const uint32_t here = !have ? 0u : walk.end - k0 < have ? static_cast<uint32_t>(walk.end - k0) : have;
+        const uint32_t live = f < n_filters ? (1u << here) - 1u : 0u;  // keys of the first filter
+        uint32_t gone = 0;
 #pragma unroll
-        for (int j = 0; j < KPT; ++j) {
-            const uint64_t k = k0 + j;
-            const bool v = k < n;
-            uint32_t f = 0;
-            bool ok = false;
-            bool live = v;
+        for (int g = 0; g < KPT; g += B) {
+            uint64_t b[B];
+            uint32_t fp[B];
+            uint64_t c[B][C::nchunks];
+#pragma unroll
+            for (int j = 0; j < B; ++j) {
+                if ((live >> (g + j)) & 1u) {
+                    candidates<C>(key[g + j], t.nb_mask, b[j], fp[j]);
+                    load_rlx<C::bucket_bytes>(bucket_words<C>(t, b[j]), c[j]);
+                }
+            }
+#pragma unroll
+            for (int j = 0; j < B; ++j)
+                if (((live >> (g + j)) & 1u) && try_remove<C>(bucket_words<C>(t, b[j]), c[j], fp[j], err)) gone |= 1u << (g + j);
+#pragma unroll
+            for (int j = 0; j < B; ++j) {
+                if (((live & ~gone) >> (g + j)) & 1u) {
+                    b[j] = alt_bucket<C>(b[j], fp[j], t.nb_mask);
+                    load_rlx<C::bucket_bytes>(bucket_words<C>(t, b[j]), c[j]);
+                }
+            }
+#pragma unroll
+            for (int j = 0; j < B; ++j)
+                if ((((live & ~gone) >> (g + j)) & 1u) && !err &&
+                    try_remove<C>(bucket_words<C>(t, b[j]), c[j], alt_tag<C>(fp[j]), err))
+                    gone |= 1u << (g + j);
+        }
+        {
+            const int32_t r = __popc(gone);
+            set_add_ctrs(descs, f, live != 0, {{CTR_REMOVED, r}, {CTR_OCCUPIED, -r}});
+        }
+        for (uint32_t j = here; __any_sync(0xFFFFFFFFu, j < have); ++j) {  // keys past the first filter
+            bool ok = false, v = j < have;
             if (v) {
-                item = set_advance(offs, n_items, item, k);
-                f = set_filter(filt, item, n_filters);
-                live = f < n_filters;
+                walk.to(offs, n_items, k0 + j);
+                f = set_filter(filt, walk.item, n_filters);
+                bad |= f == n_filters;
+                v = f < n_filters;
             }
-            if (v && !live) {
-                bad = true;
-                if (out) out[k] = 0;
-            }
-            if (live) {
-                const DevTable t = descs[f];
+            if (v) {
+                const DevTable t2 = descs[f];
                 uint64_t b;
                 uint32_t fp;
-                candidates<C>(static_cast<uint64_t>(keys[k]), t.nb_mask, b, fp);
                 uint64_t c[C::nchunks];
-                load_rlx<C::bucket_bytes>(t.buckets + b * C::bucket_bytes, c);
-                ok = try_remove<C>(bucket_words<C>(t, b), c, fp, err);
+                candidates<C>(static_cast<uint64_t>(keys[k0 + j]), t2.nb_mask, b, fp);
+                load_rlx<C::bucket_bytes>(bucket_words<C>(t2, b), c);
+                ok = try_remove<C>(bucket_words<C>(t2, b), c, fp, err);
                 if (!ok && !err) {
-                    b = alt_bucket<C>(b, fp, t.nb_mask);
-                    fp = alt_tag<C>(fp);
-                    load_rlx<C::bucket_bytes>(t.buckets + b * C::bucket_bytes, c);
-                    ok = try_remove<C>(bucket_words<C>(t, b), c, fp, err);
+                    b = alt_bucket<C>(b, fp, t2.nb_mask);
+                    load_rlx<C::bucket_bytes>(bucket_words<C>(t2, b), c);
+                    ok = try_remove<C>(bucket_words<C>(t2, b), c, alt_tag<C>(fp), err);
                 }
-                if (out) out[k] = ok ? 1 : 0;
+                gone |= (ok ? 1u : 0u) << j;
             }
-            set_add_ctr(descs, f, live, CTR_REMOVED, ok ? 1u : 0u);
+            set_add_ctrs(descs, f, v, {{CTR_REMOVED, ok ? 1 : 0}, {CTR_OCCUPIED, ok ? -1 : 0}});
         }
+        if (have && out) store_results<KPT>(out, k0, n, out_vec, gone);
     }
     if (__any_sync(0xFFFFFFFFu, err) && (threadIdx.x & 31) == 0) atomicOr(err_flag, ERR_CAS_LIMIT);
     if (bad) atomicOr(err_flag, ERR_BAD_FILTER);
@@ -247,19 +337,28 @@ __global__ void __launch_bounds__(512) k_set_delete(const DevTable* __restrict__
 // slot of the primary, else of the alternate bucket; keys whose two buckets
 // are full are parked per warp and evicted 32 at a time, one per lane (as
 // k_insert does).
+// Bound by instruction issue and by the compare-and-swaps' latency.  The same
+// 14.2 M keys took 1041 us with one bucket load in flight per thread and three
+// matched counter updates per key; 604 like this, 472 with the slot masks of
+// cf_kernels.cuh.  Two CTAs of 512 threads (64 registers, some of them spilled in
+// the eviction) beat the 128-register form, 765 us.
 template <class C, int KPT>
-__global__ void __launch_bounds__(512) k_set_insert(const DevTable* __restrict__ descs, const uint32_t* __restrict__ filt,
-                                                    const uint64_t* __restrict__ offs, uint32_t n_items, uint32_t n_filters,
-                                                    const typename C::Key* __restrict__ keys, uint64_t n,
-                                                    uint8_t* __restrict__ out, uint32_t policy_bfs, uint32_t max_ev,
-                                                    unsigned long long* err_flag) {
+__global__ void __launch_bounds__(512, 2) k_set_insert(const DevTable* __restrict__ descs, const uint32_t* __restrict__ filt,
+                                                       const uint64_t* __restrict__ offs, uint32_t n_items,
+                                                       uint32_t n_filters, const typename C::Key* __restrict__ keys, uint64_t n,
+                                                       uint8_t* __restrict__ out, uint32_t policy_bfs, uint32_t max_ev,
+                                                       unsigned long long* err_flag) {
+    constexpr int B = set_batch<KPT>();
     constexpr int kBuf = 32 + 32 * KPT;
     __shared__ uint64_t s_defer[16 * kBuf];
+    __shared__ uint32_t s_items[2];
     uint64_t* buf = s_defer + (threadIdx.x >> 5) * kBuf;
     const uint32_t lane = threadIdx.x & 31;
     uint32_t pending = 0;
     bool err = false, bad = false;
     const uint64_t tile = static_cast<uint64_t>(blockDim.x) * KPT;
+    const bool keys_vec = reinterpret_cast<uintptr_t>(keys) % (KPT * C::key_bytes < 32 ? KPT * C::key_bytes : 32) == 0;
+    const bool out_vec = reinterpret_cast<uintptr_t>(out) % KPT == 0;
 
     // evict the parked key index idx (or nothing when !v); warp-uniform call
     auto evict_parked = [&](uint64_t idx, bool v) {
@@ -268,62 +367,94 @@ __global__ void __launch_bounds__(512) k_set_insert(const DevTable* __restrict__
         EvictStats st;
         if (v) {
             // parked keys passed the filter check when they were first tried
-            f = set_filter(filt, set_find_item(offs, n_items, idx), n_filters);
+            f = set_filter(filt, set_find_item(offs, 0, n_items, idx), n_filters);
             ok = evict_key<C>(descs[f], static_cast<uint64_t>(keys[idx]), policy_bfs, max_ev, st, err);
             if (ok && out) out[idx] = 1;
         }
-        set_add_ctr(descs, f, v, CTR_EVICTED_INSERTS, 1u);
-        set_add_ctr(descs, f, v, CTR_FAILED, ok ? 0u : 1u);
-        set_add_ctr(descs, f, v, CTR_EVICTIONS, st.evictions);
-        set_add_ctr(descs, f, v, CTR_LOST, st.lost);
-        set_add_ctr(descs, f, v, CTR_DUP, st.dup);
-        set_add_ctr(descs, f, v, CTR_OCCUPIED, (ok ? 1u : 0u) - st.lost + st.dup);
+        set_add_ctrs(descs, f, v,
+                     {{CTR_EVICTED_INSERTS, 1},
+                      {CTR_FAILED, ok ? 0 : 1},
+                      {CTR_EVICTIONS, static_cast<int32_t>(st.evictions)},
+                      {CTR_LOST, static_cast<int32_t>(st.lost)},
+                      {CTR_DUP, static_cast<int32_t>(st.dup)},
+                      {CTR_OCCUPIED, static_cast<int32_t>((ok ? 1u : 0u) - st.lost + st.dup)}});
     };
 
     for (uint64_t base = blockIdx.x * tile; base < n; base += static_cast<uint64_t>(gridDim.x) * tile) {
+        set_tile_items(offs, n_items, base, (base + tile < n ? base + tile : n) - 1, s_items);
         const uint64_t k0 = base + static_cast<uint64_t>(threadIdx.x) * KPT;
-        uint32_t item = k0 < n ? set_find_item(offs, n_items, k0) : 0;
-        uint32_t hard = 0;
+        const uint32_t have = k0 < n ? (n - k0 < KPT ? static_cast<uint32_t>(n - k0) : KPT) : 0u;
+        uint64_t key[KPT];
+        if (have) load_keys<C, KPT>(keys, k0, n, keys_vec, key);
+        SetWalk walk(offs, s_items, have ? k0 : base);
+        uint32_t f = set_filter(filt, walk.item, n_filters);
+        bad |= have && f == n_filters;
+        const DevTable t = descs[f < n_filters ? f : 0];
+        const uint32_t here = !have ? 0u : walk.end - k0 < have ? static_cast<uint32_t>(walk.end - k0) : have;
+        uint32_t live = f < n_filters ? (1u << here) - 1u : 0u;  // keys of the first filter
+        uint32_t prim = 0, sec = 0;                              // one bit per key
 #pragma unroll
-        for (int j = 0; j < KPT; ++j) {
-            const uint64_t k = k0 + j;
-            const bool v = k < n;
-            uint32_t f = 0;
-            int where = 0;  // 1 primary, 2 secondary, 0 not stored
-            bool live = v;
-            if (v) {
-                item = set_advance(offs, n_items, item, k);
-                f = set_filter(filt, item, n_filters);
-                live = f < n_filters;
-                if (!live) {
-                    bad = true;
-                    if (out) out[k] = 0;
+        for (int g = 0; g < KPT; g += B) {
+            uint64_t b[B];
+            uint32_t fp[B];
+            uint64_t c[B][C::nchunks];
+#pragma unroll
+            for (int j = 0; j < B; ++j) {
+                if ((live >> (g + j)) & 1u) {
+                    candidates<C>(key[g + j], t.nb_mask, b[j], fp[j]);
+                    load_rlx<C::bucket_bytes>(bucket_words<C>(t, b[j]), c[j]);
                 }
             }
-            if (live) {
-                const DevTable t = descs[f];
+#pragma unroll
+            for (int j = 0; j < B; ++j)
+                if (((live >> (g + j)) & 1u) && try_insert<C>(bucket_words<C>(t, b[j]), c[j], fp[j], err)) prim |= 1u << (g + j);
+#pragma unroll
+            for (int j = 0; j < B; ++j) {
+                if (((live & ~prim) >> (g + j)) & 1u) {
+                    b[j] = alt_bucket<C>(b[j], fp[j], t.nb_mask);
+                    load_rlx<C::bucket_bytes>(bucket_words<C>(t, b[j]), c[j]);
+                }
+            }
+#pragma unroll
+            for (int j = 0; j < B; ++j)
+                if ((((live & ~prim) >> (g + j)) & 1u) && !err &&
+                    try_insert<C>(bucket_words<C>(t, b[j]), c[j], alt_tag<C>(fp[j]), err))
+                    sec |= 1u << (g + j);
+        }
+        {
+            const int32_t p = __popc(prim), q = __popc(sec);
+            set_add_ctrs(descs, f, live != 0, {{CTR_PRIMARY, p}, {CTR_SECONDARY, q}, {CTR_OCCUPIED, p + q}});
+        }
+        for (uint32_t j = here; __any_sync(0xFFFFFFFFu, j < have); ++j) {  // keys past the first filter
+            bool p = false, q = false, v = j < have;
+            if (v) {
+                walk.to(offs, n_items, k0 + j);
+                f = set_filter(filt, walk.item, n_filters);
+                bad |= f == n_filters;
+                v = f < n_filters;
+            }
+            if (v) {
+                const DevTable t2 = descs[f];
                 uint64_t b;
                 uint32_t fp;
-                candidates<C>(static_cast<uint64_t>(keys[k]), t.nb_mask, b, fp);
                 uint64_t c[C::nchunks];
-                load_rlx<C::bucket_bytes>(t.buckets + b * C::bucket_bytes, c);
-                if (try_insert<C>(bucket_words<C>(t, b), c, fp, err)) {
-                    where = 1;
-                } else if (!err) {
-                    b = alt_bucket<C>(b, fp, t.nb_mask);
-                    fp = alt_tag<C>(fp);
-                    load_rlx<C::bucket_bytes>(t.buckets + b * C::bucket_bytes, c);
-                    if (try_insert<C>(bucket_words<C>(t, b), c, fp, err)) where = 2;
+                candidates<C>(static_cast<uint64_t>(keys[k0 + j]), t2.nb_mask, b, fp);
+                load_rlx<C::bucket_bytes>(bucket_words<C>(t2, b), c);
+                p = try_insert<C>(bucket_words<C>(t2, b), c, fp, err);
+                if (!p && !err) {
+                    b = alt_bucket<C>(b, fp, t2.nb_mask);
+                    load_rlx<C::bucket_bytes>(bucket_words<C>(t2, b), c);
+                    q = try_insert<C>(bucket_words<C>(t2, b), c, alt_tag<C>(fp), err);
                 }
-                if (where == 0) hard |= 1u << j;
-                if (where && out) out[k] = 1;
-                if (!where && out) out[k] = 0;
+                live |= 1u << j;
+                prim |= (p ? 1u : 0u) << j;
+                sec |= (q ? 1u : 0u) << j;
             }
-            set_add_ctr(descs, f, live, CTR_PRIMARY, where == 1 ? 1u : 0u);
-            set_add_ctr(descs, f, live, CTR_SECONDARY, where == 2 ? 1u : 0u);
-            set_add_ctr(descs, f, live, CTR_OCCUPIED, where ? 1u : 0u);
+            set_add_ctrs(descs, f, v, {{CTR_PRIMARY, p ? 1 : 0}, {CTR_SECONDARY, q ? 1 : 0}, {CTR_OCCUPIED, p || q ? 1 : 0}});
         }
+        if (have && out) store_results<KPT>(out, k0, n, out_vec, prim | sec);
         // park the keys whose buckets are both full
+        const uint32_t hard = live & ~(prim | sec);
         const uint32_t cnt = __popc(hard);
         const uint32_t incl = warp_inclusive_scan(cnt);
         const uint32_t total = __shfl_sync(0xFFFFFFFFu, incl, 31);

@@ -160,3 +160,50 @@ def test_binned_insert_of_repeated_keys(cfb, orc, kb, bits, bs, slots, hot, copi
         hopeless = np.isin(c[0], full) & np.isin(c[1], full)
         assert np.all(host_u8(f.containsMany(dev(rest))).astype(bool) | hopeless)
     f.close()
+
+
+@pytest.mark.parametrize("bits,bs", [(8, 16), (16, 16), (32, 8)])
+@pytest.mark.parametrize("kpt", [1, 2, 4, 8])
+def test_set_items_that_end_inside_a_thread(cfb, orc, bits, bs, kpt):
+    """Items of 0 to 40 keys, so that a thread's keys, a warp's and a tile's belong
+    to several filters, with one item of a filter outside the set; every filter
+    ends up as its own keys inserted into the oracle would leave it."""
+    cfg = cfb.CuckooConfig(T="uint64", bitsPerTag=bits, bucketSize=bs, evictionPolicy=cfb.EvictionPolicy.BFS)
+    nf = 48
+    fs = cfb.CuckooFilterSet(cfg, [512] * nf)
+    rng = np.random.default_rng(kpt)
+    sizes = rng.choice([0, 1, 2, 3, 5, 8, 31, 33, 40], 400)
+    filt = rng.integers(0, nf, 400).astype(np.int32)
+    filt[200] = nf + 7
+    sizes[200] = 3
+    offs = np.concatenate([[0], np.cumsum(sizes)]).astype(np.int64)
+    n = int(offs[-1])
+    keys = orc.splitmix64(31, n)
+    for op in (cfb.SET_INSERT, cfb.SET_CONTAINS, cfb.SET_DELETE):
+        fs.set_launch(op, 128, kpt)
+    owner = np.repeat(filt, sizes)
+    ok = owner < nf
+    d, o, w = dev(keys), torch.from_numpy(offs).cuda(), torch.from_numpy(filt).cuda()
+    res = torch.full((n,), 7, dtype=torch.uint8, device="cuda")
+    fs.insert_async(d, o, w, res)
+    with pytest.raises(cfb.CuckooError):
+        fs.sync()
+    got = res.cpu().numpy()
+    assert np.array_equal(got, ok.astype(np.uint8))  # at most 300 keys in 512 slots: none fails
+    occ = fs.occupied()
+    for i in range(nf):
+        assert occ[i] == int((owner == i).sum()) == fs.stats(i)["occupied"]
+        assert fs.stats(i)["primary"] + fs.stats(i)["secondary"] + fs.stats(i)["evicted_inserts"] == occ[i]
+    fs.contains_async(d, o, w, res)
+    assert np.array_equal(res.cpu().numpy(), ok.astype(np.uint8))
+    half = np.arange(n) % 2 == 0  # delete the even keys, as items of the same filters
+    o2 = torch.from_numpy(np.concatenate([[0], np.cumsum(half)])[offs].astype(np.int64)).cuda()
+    gone = torch.full((int(half.sum()),), 7, dtype=torch.uint8, device="cuda")
+    fs.delete_async(dev(keys[half]), o2, w, gone)
+    assert np.array_equal(gone.cpu().numpy(), ok[half].astype(np.uint8))
+    occ = fs.occupied()
+    for i in range(nf):
+        assert occ[i] == int((owner[~half] == i).sum())
+    fs.contains_async(dev(keys[~half]), torch.from_numpy(np.concatenate([[0], np.cumsum(~half)])[offs].astype(np.int64)).cuda(),
+                      w, res[:int((~half).sum())])
+    assert np.array_equal(res[:int((~half).sum())].cpu().numpy(), ok[~half].astype(np.uint8))
