@@ -107,19 +107,46 @@ template <class C>
 using SlotMask = typename std::conditional<(C::bs > 32), unsigned long long, unsigned int>::type;
 
 // Bit s set when slot s of bucket image c holds `tag` (0: the empty slots).
+// Random inserts and deletes in an L2-resident table are bound by instruction
+// issue, and this is most of it, so it is written for each tag width: 16-bit
+// lanes are cut to 0 or 1 by a 16x2 minimum and gathered by multiply-adds (about
+// 20 instructions for 16 slots, 60 with 64-bit lane flags), 8-bit ones are
+// gathered by one multiply per four, 32-bit ones compared one by one.
 template <class C>
 __device__ __forceinline__ SlotMask<C> slots_holding(const uint64_t (&c)[C::nchunks], uint32_t tag) {
     static_assert(C::bs <= 64, "slot masks hold at most 64 slots");
-    const uint64_t rep = replicate<C::bits>(tag);
-    SlotMask<C> m = 0;
+    using M = SlotMask<C>;
+    M other = 0;  // slots holding anything else
+    if constexpr (C::bits == 16) {
+        const uint32_t rep = tag * 0x00010001u;
+        constexpr int G = C::nchunks < 4 ? C::nchunks : 4;  // chunks of a group of up to 16 slots
 #pragma unroll
-    for (int j = 0; j < C::nchunks; ++j) {
-        const uint64_t z = zero_lanes<C::bits>(c[j] ^ rep);
+        for (int g = 0; g < C::nchunks; g += G) {
+            uint32_t acc = 0;  // slot 2k of the group at bit 2k, slot 2k + 1 at bit 16 + 2k
 #pragma unroll
-        for (int l = 0; l < C::lanes_per_chunk; ++l)
-            m |= static_cast<SlotMask<C>>((z >> (l * C::bits + C::bits - 1)) & 1u) << (j * C::lanes_per_chunk + l);
+            for (int j = 0; j < G; ++j) {
+                const uint32_t lo = __vimin3_u16x2(static_cast<uint32_t>(c[g + j]) ^ rep, 0x00010001u, 0x00010001u);
+                const uint32_t hi = __vimin3_u16x2(static_cast<uint32_t>(c[g + j] >> 32) ^ rep, 0x00010001u, 0x00010001u);
+                acc += lo * (1u << (4 * j)) + hi * (4u << (4 * j));
+            }
+            other |= static_cast<M>((acc | acc >> 15) & 0xFFFFu) << (4 * g);
+        }
+    } else if constexpr (C::bits == 8) {
+        const uint32_t rep = tag * 0x01010101u;
+#pragma unroll
+        for (int j = 0; j < 2 * C::nchunks; ++j) {
+            const uint32_t x = static_cast<uint32_t>(c[j / 2] >> (32 * (j % 2))) ^ rep;
+            const uint32_t t = ((((x & 0x7F7F7F7Fu) + 0x7F7F7F7Fu) | x) >> 7) & 0x01010101u;  // 1 per lane that differs
+            // lane flags 0, 8, 16, 24 to bits 24..27: no two products meet below them
+            other |= static_cast<M>((t * 0x01020408u) >> 24) << (4 * j);
+        }
+    } else {
+#pragma unroll
+        for (int j = 0; j < 2 * C::nchunks; ++j)
+            other |= static_cast<M>(static_cast<uint32_t>(c[j / 2] >> (32 * (j % 2))) != tag ? 1u : 0u) << j;
     }
-    return m;
+    constexpr M full = C::bs == 8 * sizeof(M) ? ~static_cast<M>(0) : ((static_cast<M>(1) << (C::bs % (8 * sizeof(M)))) - 1);
+    return other ^ full;
 }
 
 // First slot set in m, circularly from slot s0 (m != 0).
@@ -145,10 +172,11 @@ __device__ __forceinline__ uint32_t scan_slot(SlotMask<C> m, uint32_t tag) {
 }
 
 // tryInsertAtBucket on a bucket whose current image is in c (refreshed on
-// compare-and-swap failure).  Returns true when fp was stored.
+// compare-and-swap failure).  Returns true when fp was stored.  Buckets of up to
+// 64 slots are scanned by slot mask; of 128 (64-bit words only) word by word.
 template <class C>
 __device__ bool try_insert(uint64_t* bw, uint64_t (&c)[C::nchunks], uint32_t fp, bool& err) {
-    if constexpr (!C::chunk_scan) {
+    if constexpr (C::bs <= 64) {
         for (int it = 0; it < kCasRetryLimit; ++it) {
             const SlotMask<C> m = slots_holding<C>(c, 0);
             if (!m) return false;
@@ -187,7 +215,7 @@ __device__ bool try_insert(uint64_t* bw, uint64_t (&c)[C::nchunks], uint32_t fp,
 template <class C>
 __device__ __forceinline__ bool plan_insert(const uint64_t (&c)[C::nchunks], uint32_t fp, int& w, uint64_t& cur,
                                             uint64_t& desired) {
-    if constexpr (!C::chunk_scan) {
+    if constexpr (C::bs <= 64) {
         const SlotMask<C> m = slots_holding<C>(c, 0);
         if (!m) return false;
         const uint32_t slot = scan_slot<C>(m, fp);
@@ -215,7 +243,7 @@ template <class C>
 __device__ __forceinline__ bool plan_remove(const uint64_t (&c)[C::nchunks], uint32_t fp, int& w, uint64_t& cur,
                                             uint64_t& desired) {
     constexpr uint64_t lane_mask = C::bits == 32 ? 0xFFFFFFFFULL : ((1ULL << C::bits) - 1ULL);
-    if constexpr (!C::chunk_scan) {
+    if constexpr (C::bs <= 64) {
         const SlotMask<C> m = slots_holding<C>(c, fp);
         if (!m) return false;
         const uint32_t slot = scan_slot<C>(m, fp);
@@ -241,7 +269,7 @@ __device__ __forceinline__ bool plan_remove(const uint64_t (&c)[C::nchunks], uin
 template <class C>
 __device__ bool try_remove(uint64_t* bw, uint64_t (&c)[C::nchunks], uint32_t fp, bool& err) {
     constexpr uint64_t lane_mask = C::bits == 32 ? 0xFFFFFFFFULL : ((1ULL << C::bits) - 1ULL);
-    if constexpr (!C::chunk_scan) {
+    if constexpr (C::bs <= 64) {
         for (int it = 0; it < kCasRetryLimit; ++it) {
             const SlotMask<C> m = slots_holding<C>(c, fp);
             if (!m) return false;

@@ -84,7 +84,10 @@ constexpr uint32_t kRound1SlackSixteenths = 3;
 // tags 45.4 -> 130.4 in 64 MiB, 32.6 -> 41.9 in 256 MiB; from 512 MiB on
 // within 2 %).
 constexpr int kContainsKPT = 2;
-constexpr int kDeleteKPT = 4;
+// Deletes likewise: 63 registers against 114 (31 K to 33 M deletes, us at 4 -> 2:
+// 26.7 -> 19.6 and 71.5 -> 56.5 in 2 and 32 MiB, 212.9 -> 201.2 in 128 MiB, 1010 -> 993
+// in 2 GiB; only 16-byte buckets past L2 prefer 4, 273 -> 305 in 256 MiB).
+constexpr int kDeleteKPT = 2;
 constexpr int kInsertKPT = 2;
 
 enum KernelId : int { KID_CONTAINS = 0, KID_DELETE = 1, KID_INSERT = 2, KID_COUNT_KERNELS = 3 };
