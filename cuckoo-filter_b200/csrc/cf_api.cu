@@ -85,9 +85,9 @@ int cuda_fail(cudaError_t e, const char* what) {
 const std::vector<OpsTable>& registry() {
     static std::vector<OpsTable> v = [] {
         std::vector<OpsTable> r;
-        register_bits8(r);
-        register_bits16(r);
-        register_bits32(r);
+        for (auto* add : {register_bits8, register_bits8_more, register_bits16, register_bits16_more,
+                          register_bits16_policy, register_bits32, register_bits32_more})
+            add(r);
         return r;
     }();
     return v;
@@ -425,7 +425,7 @@ bool bin_geometry(const cf_filter* f, uint64_t m, BinGeom* g) {
     g->l2 = l2;
     g->nseg = static_cast<uint32_t>(nseg);
     g->d1 = static_cast<uint32_t>(((nseg - 1) >> l2) + 1);
-    g->entry_bytes2 = bits < 32 && sbl + bits <= 32 ? 4 : 8;
+    g->entry_bytes2 = bits < 32 ? 4 : 8;  // (at most 13 bits of bucket: 64 KiB of 8-byte buckets)
     g->entry_bytes1 = g->entry_bytes2 == 4 && l2 + sbl + bits <= 32 ? 4 : 8;
     // Room of a bin: the mean of evenly hashed keys plus six standard deviations
     // (the AddSub policy's primary buckets are the first half of the table).
@@ -496,14 +496,14 @@ int run_binned(cf_filter* f, const void* keys, uint64_t n, uint8_t* out, void* s
         w.pay[1] = reinterpret_cast<uint32_t*>(p + al(room * 4) + al(g.ent[0] * 4));
         p += pays;
     }
-    w.cursor = reinterpret_cast<uint32_t*>(p);
-    p += al(cursors);
     w.left = reinterpret_cast<uint32_t*>(p);
     p += al(g.nseg * 4ull);
+    w.cursor = reinterpret_cast<uint32_t*>(p);
+    p += al(cursors);
     w.cnt = reinterpret_cast<unsigned long long*>(p);
     p += al(64);
-    w.full_words = words;
     w.full = words ? reinterpret_cast<uint32_t*>(p) : nullptr;
+    w.zero_bytes = al(cursors) + al(64) + words * 4;
     w.list_room = room;
     w.h_cnt = f->h_cnt;
     w.sms = f->sms;

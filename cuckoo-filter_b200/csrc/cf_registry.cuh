@@ -73,6 +73,9 @@ constexpr int kRgGatherMaxSmem = 160 * 1024;
 // The eviction kernels run this many waves of CTAs (each warp takes an equal
 // share of the list; more, smaller shares were measured faster on B200).
 constexpr int kEvictGridWaves = 4;
+// Batch size up to which a binned insert evicts with NC lanes per key (see
+// k_evict_bfs_coop; the lockstep pass overtook it between 32 M and 64 M keys).
+constexpr uint64_t kCoopEvictBatch = 1ull << 25;
 // Slots of each bucket (in sixteenths) that the first round of a large
 // segment-staged insert leaves free for the second round.
 constexpr uint32_t kRound1SlackSixteenths = 3;
@@ -460,12 +463,21 @@ struct Launchers {
                            uint64_t* rest, uint32_t* rest_pay, unsigned long long* rest_count,
                            unsigned long long* dfs_count, uint32_t* bitmap, uint8_t* fail_out, uint32_t* full, int sms,
                            cudaStream_t s, uint32_t policy_bfs, uint32_t max_ev,
-                           const unsigned long long* first = nullptr) {
+                           const unsigned long long* first = nullptr, uint64_t batch = UINT64_MAX) {
         static const int list_bps = blocks_per_sm(k_evict_list<C>, 256, 0);
         if (!policy_bfs) {
             { k_evict_list<C><<<sms * list_bps * kEvictGridWaves, 256, 0, s>>>(t, list, list_pay, count, 0u, max_ev, bitmap,
                                                                               0u, fail_out, first); CF_COUNT_LAUNCH(); }
             return;
+        }
+        if constexpr (C::bs <= 16) {
+            if (!bitmap && batch <= kCoopEvictBatch) {
+                { k_evict_bfs_coop<C><<<sms * 4, 256, 0, s>>>(t, list, list_pay, count, first, rest, rest_pay, dfs_count, full);
+                  CF_COUNT_LAUNCH(); }
+                { k_evict_list<C><<<sms * 2, 256, 0, s>>>(t, rest, rest_pay, dfs_count, 0u, max_ev, bitmap, 1u, fail_out,
+                                                          nullptr); CF_COUNT_LAUNCH(); }
+                return;
+            }
         }
         static const int fast_bps = blocks_per_sm(k_evict_bfs_fast<C, kBfsFastProbes>, 256, 0);
         static const int bfs_bps = blocks_per_sm(k_evict_bfs_steps<C>, 256, 0);
@@ -520,9 +532,7 @@ struct Launchers {
         const uint32_t cap1 = w.round1_cap ? w.round1_cap : m >= t.nb_mask + 1 ? round1_cap() : C::bs;
         const int rounds = cap1 < static_cast<uint32_t>(C::bs) ? 3 : 2;
         const uint32_t per_round = ((g.l2 ? g.d1 : 0u) + g.nseg) * kCursorStride;
-        cudaError_t e = cudaMemsetAsync(w.cnt, 0, 8 * sizeof(unsigned long long), s);
-        if (e == cudaSuccess) e = cudaMemsetAsync(w.cursor, 0, sizeof(uint32_t) * per_round * rounds, s);
-        if (e == cudaSuccess && w.full) e = cudaMemsetAsync(w.full, 0, w.full_words * sizeof(uint32_t), s);
+        cudaError_t e = cudaMemsetAsync(w.cursor, 0, w.zero_bytes, s);
         if (e == cudaSuccess && PAY) e = cudaMemsetAsync(out, 1, m, s);  // failed keys are cleared at the end
         const int smem = static_cast<int>((static_cast<size_t>(C::bucket_bytes) + 4) << g.sbl);
         constexpr int kMaxSmem = kSegBytes + kSegBytes / C::bucket_bytes * 4;
@@ -609,7 +619,7 @@ struct Launchers {
         { k_bin_over<C><<<w.sms * 2, 256, 0, s>>>(t, w.list, w.list_pay, &w.cnt[0], policy_bfs, max_ev,
                                                  PAY ? out : nullptr); CF_COUNT_LAUNCH(); }
         evict_left(t, w.list, w.list_pay, &w.cnt[3], w.list + m, PAY ? w.list_pay + m : nullptr, &w.cnt[1], &w.cnt[2],
-                   nullptr, PAY ? out : nullptr, w.full, w.sms, s, policy_bfs, max_ev, &w.cnt[0]);
+                   nullptr, PAY ? out : nullptr, w.full, w.sms, s, policy_bfs, max_ev, &w.cnt[0], m);
         return cudaGetLastError();
     }
     static cudaError_t bin_insert(const DevTable& t, const BinGeom& g, const BinWork& w, const void* keys, uint64_t m,
@@ -621,10 +631,11 @@ struct Launchers {
                 return out ? bin_insert_t<decltype(e1), decltype(e2), true>(t, g, w, keys, m, out, s, policy_bfs, max_ev, skewed)
                            : bin_insert_t<decltype(e1), decltype(e2), false>(t, g, w, keys, m, out, s, policy_bfs, max_ev, skewed);
             };
-            if constexpr (C::bits < 32) {
-                if (g.entry_bytes2 == 4) return g.entry_bytes1 == 4 ? go(uint32_t{}, uint32_t{}) : go(uint64_t{}, uint32_t{});
-            }
-            return go(uint64_t{}, uint64_t{});
+            // an entry of a segment's bin fits 32 bits unless the tag alone takes them
+            if constexpr (C::bits < 32)
+                return g.entry_bytes1 == 4 ? go(uint32_t{}, uint32_t{}) : go(uint64_t{}, uint32_t{});
+            else
+                return go(uint64_t{}, uint64_t{});
         }
     }
 
@@ -832,9 +843,13 @@ struct Launchers {
     }
 };
 
-// Registration hooks, one per translation unit (tag width).
+// Registration hooks, one per translation unit (they compile side by side).
 void register_bits8(std::vector<OpsTable>& v);
+void register_bits8_more(std::vector<OpsTable>& v);
 void register_bits16(std::vector<OpsTable>& v);
+void register_bits16_more(std::vector<OpsTable>& v);
+void register_bits16_policy(std::vector<OpsTable>& v);
 void register_bits32(std::vector<OpsTable>& v);
+void register_bits32_more(std::vector<OpsTable>& v);
 
 }  // namespace cfb

@@ -1023,6 +1023,110 @@ __global__ void __launch_bounds__(256, C::nchunks <= 4 ? 3 : 2) k_evict_bfs_fast
     if (__any_sync(0xFFFFFFFFu, err) && lane == 0) atomicOr(&t.ctr[CTR_ERROR], ERR_CAS_LIMIT);
 }
 
+// BFS eviction of a short list: NC lanes per key, each probing one candidate's
+// alternate bucket, so that a key waits for four round trips (start bucket,
+// alternate buckets, copy, swap) whatever its candidates hold; the first
+// candidate in the reference's order (CuckooFilter.cuh:967-1018) with room is
+// moved, as when they are probed one after the other.  A lost race starts the
+// key over; keys whose candidates all fail, or that lose kCoopTries times, go
+// to `dfs`.  Too many probes for a long list (eight per key where the lockstep
+// pass makes about two), but a short one is bound by the longest chain: 11 and
+// 37 us in the lockstep pass and the step machine of a 2^20-slot fill, 17 here.
+// Whole fills to 0.95, us, lockstep against this: 2^14 slots 93 and 76, 2^20 139
+// and 110, 2^24 387 and 352, 2^25 711 and 689, 2^26 1232 and 1261.
+constexpr int kCoopTries = 16;
+template <class C>
+__global__ void __launch_bounds__(256) k_evict_bfs_coop(DevTable t, const uint64_t* ent, const uint32_t* pay,
+                                                        const unsigned long long* n_dev,
+                                                        const unsigned long long* first_dev, uint64_t* dfs,
+                                                        uint32_t* dfs_pay, unsigned long long* dfs_count,
+                                                        const uint32_t* full) {
+    constexpr uint64_t lane_mask = C::bits == 32 ? 0xFFFFFFFFULL : ((1ULL << C::bits) - 1ULL);
+    constexpr uint32_t NC = (C::bs / 2) < 8 ? (C::bs / 2) : 8;
+    static_assert(NC >= 1 && 32 % NC == 0, "a group of NC lanes per key");
+    const uint32_t lane = threadIdx.x & 31, q = lane % NC;
+    const uint32_t gmask = (NC == 32 ? 0xFFFFFFFFu : (1u << NC) - 1u) << (lane - q);
+    const uint64_t m = *n_dev, first = first_dev ? *first_dev : 0ull;
+    uint32_t n_evk = 0, n_ok = 0, n_ev = 0, n_dup = 0;
+    bool err = false;
+    const uint64_t step = static_cast<uint64_t>(gridDim.x) * (blockDim.x / NC);
+    // the trip count is uniform over the CTA: every lane reaches every vote
+    for (uint64_t base = static_cast<uint64_t>(blockIdx.x) * (blockDim.x / NC); base < m; base += step) {
+        const uint64_t i = base + threadIdx.x / NC;
+        const bool v = i < m;
+        bool pend = v, done = false;
+        uint64_t start = 0;
+        uint32_t fp = 0;
+        const uint64_t e = v ? ent[first + i] : 0ull;
+        if (v) {
+            n_evk += q == 0;
+            const uint32_t fp0 = static_cast<uint32_t>(e) & C::tag_mask;
+            const uint64_t i2 = e >> C::bits;
+            const bool even = (fp0 & 1u) == 0;
+            start = even ? alt_bucket<C>(i2, fp0, t.nb_mask) : i2;
+            fp = even ? alt_tag<C>(fp0) : fp0;  // the tag in the start bucket's form
+        }
+        const uint32_t slot = static_cast<uint32_t>((static_cast<uint64_t>(fp) + 7ull * q) & (C::bs - 1));
+        const int sw = static_cast<int>(slot / C::lanes_per_chunk);
+        const int sh = static_cast<int>(slot % C::lanes_per_chunk) * C::bits;
+        uint64_t* sbw = bucket_words<C>(t, start);
+        for (int tries = 0; tries < kCoopTries && __any_sync(0xFFFFFFFFu, pend); ++tries) {
+            uint64_t snap[C::nchunks], img[C::nchunks];
+            uint64_t word = 0, ab = start, exp = 0, des = 0;
+            uint32_t cand = 1;
+            int w = 0;
+            bool room = false;
+            if (pend) {
+                load_rlx<C::bucket_bytes>(sbw, snap);
+                word = pick(snap, sw);
+                cand = static_cast<uint32_t>((word >> sh) & lane_mask);
+                if (cand == 0) {
+                    room = true;
+                } else {
+                    ab = alt_bucket<C>(start, cand, t.nb_mask);
+                    if (!known_full(full, ab)) {
+                        load_rlx<C::bucket_bytes>(bucket_words<C>(t, ab), img);
+                        room = plan_insert<C>(img, alt_tag<C>(cand), w, exp, des);
+                    }
+                }
+            }
+            const uint32_t vote = __ballot_sync(0xFFFFFFFFu, room) & gmask;
+            if (pend && vote == 0) pend = false;  // no candidate can move: BFS is over
+            bool stored = false;
+            if (pend && lane == static_cast<uint32_t>(__ffs(vote) - 1)) {
+                if (cand == 0) {  // reference :980-985: a free slot, insert fp into the start bucket
+                    stored = try_insert<C>(sbw, snap, fp, err);
+                    if (stored) record_chain(t, 0u);
+                } else if (cas64(bucket_words<C>(t, ab) + w, exp, des) == exp) {  // the candidate is copied
+                    const uint64_t swapped = (word & ~(lane_mask << sh)) | (static_cast<uint64_t>(fp) << sh);
+                    stored = cas64(sbw + sw, word, swapped) == word;
+                    if (stored) {
+                        ++n_ev;
+                        record_chain(t, 1u);
+                    } else if (!remove_from_pair<C>(t, ab, start, alt_tag<C>(cand), err)) {
+                        ++n_dup;  // the copy could not be taken back: an extra entry
+                    }
+                }
+            }
+            if ((__ballot_sync(0xFFFFFFFFu, stored) & gmask) != 0) {
+                done = true;
+                pend = false;
+            }
+        }
+        if (done) n_ok += q == 0;
+        if (v && !done && q == 0) {
+            const unsigned long long o = atomicAdd(dfs_count, 1ull);
+            dfs[o] = e;
+            if (dfs_pay) dfs_pay[o] = pay[first + i];
+        }
+    }
+    flush_counters(t.ctr, {{CTR_OCCUPIED, static_cast<int32_t>(n_ok + n_dup)},
+                           {CTR_DUP, static_cast<int32_t>(n_dup)},
+                           {CTR_EVICTED_INSERTS, static_cast<int32_t>(n_evk)},
+                           {CTR_EVICTIONS, static_cast<int32_t>(n_ev)}});
+    if (__any_sync(0xFFFFFFFFu, err) && lane == 0) atomicOr(&t.ctr[CTR_ERROR], ERR_CAS_LIMIT);
+}
+
 // Eviction for the keys whose two buckets were full after both segment rounds
 // (or, with `continued`, whose BFS candidates all failed); entries carry
 // (alternate bucket, tag).  One key per thread, all lanes busy.  Results: a

@@ -207,3 +207,33 @@ def test_set_items_that_end_inside_a_thread(cfb, orc, bits, bs, kpt):
     fs.contains_async(dev(keys[~half]), torch.from_numpy(np.concatenate([[0], np.cumsum(~half)])[offs].astype(np.int64)).cuda(),
                       w, res[:int((~half).sum())])
     assert np.array_equal(res[:int((~half).sum())].cpu().numpy(), ok[~half].astype(np.uint8))
+
+
+@pytest.mark.parametrize("kb,bits,bs,load", [(8, 16, 16, 0.99), (4, 8, 16, 0.98), (8, 8, 8, 0.95), (8, 32, 8, 0.97),
+                                             (8, 16, 4, 0.93), (8, 32, 2, 0.86)])
+def test_short_eviction_lists(cfb, orc, kb, bits, bs, load):
+    """A fill past the load where keys begin to fail, with as many eviction lanes
+    per key as the geometry has candidates: flags, counters, chain histogram and
+    table agree, and every stored key can be taken out again."""
+    cfg = cfb.CuckooConfig(T="uint64" if kb == 8 else "uint32", bitsPerTag=bits, bucketSize=bs, maxEvictions=200,
+                           evictionPolicy=cfb.EvictionPolicy.BFS)
+    f = cfb.CuckooFilter(cfg, 1 << 18)
+    f.setOption(cfb.OPT_CHAIN_HISTOGRAM, 1)
+    keys = orc.splitmix64(61 + bits + bs, int(load * f.capacity()))
+    if kb == 4:
+        keys = keys.astype(np.uint32)
+    d = dev(keys)
+    ok = torch.zeros(len(keys), dtype=torch.bool, device="cuda")
+    occ = f.insertMany(d, d_output=ok)
+    st = f.stats()
+    stored = int(ok.sum())
+    assert stored == len(keys) - st["failed"]
+    assert occ == f.countOccupiedSlots() == stored - st["lost"] + st["duplicates"]
+    assert st["evicted_inserts"] > 0 and st["evictions"] > 0
+    assert int(f.chainHistogram().sum()) == st["evicted_inserts"] - st["failed"]
+    if st["lost"] == st["duplicates"] == 0:
+        assert bool(f.containsMany(d[ok]).all())
+        gone = torch.zeros(stored, dtype=torch.bool, device="cuda")
+        assert f.deleteMany(d[ok], gone) == 0 and bool(gone.all())
+        assert int(f.table_image().to(torch.int32).sum()) == 0
+    f.close()
