@@ -368,16 +368,25 @@ uint64_t auto_threshold(const cf_filter* f, int op) {
     return f->num_buckets * 8;
 }
 
-// Batch size from which a batch is segment-staged.  Inserts: one key per
-// bucket (on B200 the segment path overtook random inserts between 0.5 and 1
-// key per bucket: 0.70 against 0.88 ms at 1, 0.98 against 1.73 ms at 2, on an
-// empty 2^28-slot table); deletes: eight keys per bucket.  Lookups: never.
+// Batch size from which a batch is staged.  Inserts: one key per bucket, and
+// enough keys to pay for a dozen launches: 2^17, or 2^20 for batches that cannot
+// fill the table beyond three quarters (fewer evictions, which random inserts
+// pay most for).  Binned against random, us, 16-bit tags, filling an empty table:
+// 2^14 slots to 0.95 80 and 58, to 0.6 52 and 25; 2^17 to 0.6 60 and 28; 2^20 to 0.6
+// 66 and 40, to 0.95 107 and 110; 2^22 to 0.6 80 and 92, to 0.95 156 and 236.
+// Below one key per bucket random inserts win at every size (2^26 8-bit slots,
+// 0.76 keys per bucket: 105 us a batch in the first half of the fill, 170 in the
+// second, against 309 and 382 segment-staged).
+// Deletes: eight keys per bucket.  Lookups: never.
 // Random lookups were faster for every table and batch measured (256 KiB to
 // 2 GiB, 2 to 64 keys per bucket, random against segment-staged G/s: 97 and 21
 // in 8 MiB, 65 and 25 in 128 MiB, 36 and 24 in 512 MiB, 31.4 and 21.7 in 2 GiB).
-uint64_t segmented_threshold(const cf_filter* f, int op) {
+uint64_t segmented_threshold(const cf_filter* f, int op, uint64_t n) {
     if (f->seg_min_keys) return f->seg_min_keys;
-    return op == SEG_INSERT ? f->num_buckets : op == SEG_DELETE ? f->num_buckets * 8 : UINT64_MAX;
+    if (op == SEG_DELETE) return f->num_buckets * 8;
+    if (op != SEG_INSERT) return UINT64_MAX;
+    const bool to_high_load = n >= f->num_buckets * f->cfg.bucket_size / 4 * 3;
+    return std::max<uint64_t>(f->num_buckets, to_high_load ? 1ull << 17 : 1ull << 20);
 }
 
 int run_segmented(cf_filter* f, int op, const void* keys, uint64_t n, uint8_t* out, void* stream) {
@@ -566,7 +575,7 @@ Path choose_path(const cf_filter* f, int op, uint64_t n, bool sorted_insert) {
     }
     if (f->rg_ok && n >= region_threshold(f, op)) return PATH_REGION;
     if (sorted_insert) return PATH_SEGMENT;
-    if (n >= segmented_threshold(f, op)) return PATH_SEGMENT;
+    if (n >= segmented_threshold(f, op, n)) return PATH_SEGMENT;
     return PATH_RANDOM;
 }
 

@@ -203,8 +203,9 @@ typedef enum cf_option {
     /* Batch size from which insertMany, containsMany and deleteMany stream
      * table segments through shared memory instead of probing at random
      * (insertManySorted always does).  0 = automatic: one key per bucket for
-     * inserts, eight per bucket for deletes, never for lookups (random probes
-     * were faster at every size); UINT64_MAX = never. */
+     * inserts and at least 2^17 keys (2^20 when they cannot fill the table beyond
+     * three quarters), eight per bucket for deletes, never for lookups (random
+     * probes were faster at every size); UINT64_MAX = never. */
     CF_OPT_SEGMENTED_MIN_KEYS = 2,
     /* Read-only: bytes of workspace currently allocated. */
     CF_OPT_WORKSPACE_BYTES = 3,

@@ -237,3 +237,22 @@ def test_short_eviction_lists(cfb, orc, kb, bits, bs, load):
         assert f.deleteMany(d[ok], gone) == 0 and bool(gone.all())
         assert int(f.table_image().to(torch.int32).sum()) == 0
     f.close()
+
+
+@pytest.mark.parametrize("n", [(1 << 17) - 1, 1 << 17, (1 << 20) - 1, 1 << 20])
+@pytest.mark.parametrize("load", [0.5, 0.8])
+def test_insertMany_route_by_batch_size(cfb, orc, n, load):
+    """Around the batch sizes where insertMany changes from random probes to
+    binning, for batches that fill the table beyond three quarters and not."""
+    cfg = cfb.CuckooConfig(T="uint64", bitsPerTag=16, bucketSize=16, AltBucketPolicy=POLICY["offset"],
+                           evictionPolicy=cfb.EvictionPolicy.BFS)
+    f = cfb.CuckooFilter(cfg, int(n / load))
+    keys = orc.splitmix64(71, n)
+    before = cfb.launch_count()
+    f.insertMany(dev(keys))
+    launches = cfb.launch_count() - before
+    staged = n >= (1 << 17 if load > 0.75 else 1 << 20)
+    assert (launches >= 8) == staged and (launches <= 2) == (not staged), launches
+    f.clear()
+    filled_and_emptied(cfb, f, [dev(keys)], False)
+    f.close()
