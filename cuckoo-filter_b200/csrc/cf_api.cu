@@ -8,6 +8,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
@@ -19,6 +20,10 @@
 
 using namespace cfb;
 
+// Synchronous calls on one filter that may be in flight at a time (one host
+// thread each) before two share a row of published counters.
+constexpr unsigned int kPubSlots = 64;
+
 struct cf_filter {
     cf_config cfg;
     const OpsTable* ops;
@@ -27,6 +32,11 @@ struct cf_filter {
     uint8_t* d_table;
     unsigned long long* d_ctr;  // CTR_COUNT device counters
     unsigned long long* h_ctr;  // pinned mirror
+    // Counters as the last CTA of a synchronous random insert or delete leaves
+    // them: kPubSlots rows of kPublished, one per call in flight, and the rows' tickets.
+    unsigned long long* h_pub;
+    unsigned int* d_ticket;
+    std::atomic<unsigned int> pub_next;
     int device;
     int block;
     int max_grid[KID_COUNT_KERNELS];
@@ -185,18 +195,40 @@ int check_batch(const cf_filter* f, const void* keys, uint64_t n) {
     return CF_OK;
 }
 
+int check_counters(const unsigned long long* c, uint64_t* occupied_out) {
+    if (c[CTR_ERROR] & ERR_CAS_LIMIT)
+        return fail(CF_ERR_DEVICE, "a compare-and-swap retry bound was hit on the device");
+    if (c[CTR_ERROR] & ERR_WAIT_LIMIT)
+        return fail(CF_ERR_DEVICE, "a bulk copy did not complete within its poll bound on the device");
+    if (occupied_out) *occupied_out = c[CTR_OCCUPIED];
+    return CF_OK;
+}
+
 // Synchronize, read the counters, surface device-side errors.
 int finish(cf_filter* f, void* stream, uint64_t* occupied_out) {
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     CF_CUDA(cudaMemcpyAsync(f->h_ctr, f->d_ctr, CTR_COUNT * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s),
             "counter read-back");
     CF_CUDA(cudaStreamSynchronize(s), "stream synchronize");
-    if (f->h_ctr[CTR_ERROR] & ERR_CAS_LIMIT)
-        return fail(CF_ERR_DEVICE, "a compare-and-swap retry bound was hit on the device");
-    if (f->h_ctr[CTR_ERROR] & ERR_WAIT_LIMIT)
-        return fail(CF_ERR_DEVICE, "a bulk copy did not complete within its poll bound on the device");
-    if (occupied_out) *occupied_out = f->h_ctr[CTR_OCCUPIED];
-    return CF_OK;
+    return check_counters(f->h_ctr, occupied_out);
+}
+
+// The same after a random insert or delete launched with `t`, whose last CTA
+// wrote the counters to t.pub.
+int finish_published(const DevTable& t, void* stream, uint64_t* occupied_out) {
+    CF_CUDA(cudaStreamSynchronize(static_cast<cudaStream_t>(stream)), "stream synchronize");
+    unsigned long long c[kPublished];
+    for (int i = 0; i < kPublished; ++i) c[i] = static_cast<volatile unsigned long long*>(t.pub)[i];
+    return check_counters(c, occupied_out);
+}
+
+// The table with a row of published counters of this call's own.
+DevTable dev_published(cf_filter* f) {
+    DevTable t = dev(f);
+    const unsigned int slot = f->pub_next.fetch_add(1, std::memory_order_relaxed) % kPubSlots;
+    t.pub = f->h_pub + slot * kPublished;
+    t.ticket = f->d_ticket + slot;
+    return t;
 }
 
 int ilog2(uint64_t v) { return 63 - __builtin_clzll(v); }
@@ -579,9 +611,9 @@ Path choose_path(const cf_filter* f, int op, uint64_t n, bool sorted_insert) {
     return PATH_RANDOM;
 }
 
-int do_insert(cf_filter* f, const void* keys, uint64_t n, uint8_t* out, void* stream) {
+int do_insert(cf_filter* f, const DevTable& t, const void* keys, uint64_t n, uint8_t* out, void* stream) {
     f->known_empty = false;
-    CF_CUDA(f->ops->insert(dev(f), keys, n, out, launch(f, KID_INSERT, stream),
+    CF_CUDA(f->ops->insert(t, keys, n, out, launch(f, KID_INSERT, stream),
                            f->cfg.eviction_policy == CF_EVICT_BFS ? 1u : 0u, f->cfg.max_evictions),
             "insert launch");
     return CF_OK;
@@ -697,10 +729,14 @@ int cf_create(const cf_config* cfg, uint64_t capacity, cf_filter** out) {
     f->ws_limit = 0;  // automatic
     if (e == cudaSuccess) e = cudaHostAlloc(&f->h_cnt, 4 * sizeof(unsigned long long), cudaHostAllocDefault);
     if (e == cudaSuccess) e = cudaMalloc(&f->d_table, f->table_bytes);
-    if (e == cudaSuccess) e = cudaMalloc(&f->d_ctr, CTR_COUNT * sizeof(unsigned long long));
-    if (e == cudaSuccess) e = cudaHostAlloc(&f->h_ctr, CTR_COUNT * sizeof(unsigned long long), cudaHostAllocDefault);
+    constexpr size_t kCtrBytes = CTR_COUNT * sizeof(unsigned long long) + kPubSlots * sizeof(unsigned int);
+    if (e == cudaSuccess) e = cudaMalloc(&f->d_ctr, kCtrBytes);
+    if (e == cudaSuccess) f->d_ticket = reinterpret_cast<unsigned int*>(f->d_ctr + CTR_COUNT);
+    if (e == cudaSuccess)
+        e = cudaHostAlloc(&f->h_ctr, (CTR_COUNT + kPubSlots * kPublished) * sizeof(unsigned long long), cudaHostAllocDefault);
+    if (e == cudaSuccess) f->h_pub = f->h_ctr + CTR_COUNT;
     if (e == cudaSuccess) e = cudaMemset(f->d_table, 0, f->table_bytes);
-    if (e == cudaSuccess) e = cudaMemset(f->d_ctr, 0, CTR_COUNT * sizeof(unsigned long long));
+    if (e == cudaSuccess) e = cudaMemset(f->d_ctr, 0, kCtrBytes);
     if (e == cudaSuccess) e = cudaDeviceSynchronize();
     if (e != cudaSuccess) {
         int s = cuda_fail(e, "filter allocation");
@@ -750,7 +786,7 @@ int insert_any(cf_filter* f, const void* keys, uint64_t n, uint8_t* out, void* s
                 if (int st = run_binned(f, keys, n, out, stream, &taken)) return st;
             return taken ? CF_OK : run_segmented(f, SEG_INSERT, keys, n, out, stream);
         }
-        default: return do_insert(f, keys, n, out, stream);
+        default: return do_insert(f, dev(f), keys, n, out, stream);
     }
 }
 
@@ -763,6 +799,11 @@ int cf_insert_async(cf_filter* f, const void* d_keys, uint64_t n, uint8_t* d_out
 int cf_insert(cf_filter* f, const void* d_keys, uint64_t n, uint8_t* d_out, void* stream, uint64_t* occupied_out) {
     if (int s = check_batch(f, d_keys, n)) return s;
     DeviceGuard g(f->device);
+    if (n && choose_path(f, SEG_INSERT, n, false) == PATH_RANDOM) {
+        const DevTable t = dev_published(f);
+        if (int s = do_insert(f, t, d_keys, n, d_out, stream)) return s;
+        return finish_published(t, stream, occupied_out);
+    }
     if (int s = insert_any(f, d_keys, n, d_out, stream, false)) return s;
     return finish(f, stream, occupied_out);
 }
@@ -799,6 +840,13 @@ int cf_contains(cf_filter* f, const void* d_keys, uint64_t n, uint8_t* d_out, vo
     return CF_OK;
 }
 
+int do_delete(cf_filter* f, const DevTable& t, const void* keys, uint64_t n, uint8_t* out, void* stream) {
+    LaunchCfg L = launch(f, KID_DELETE, stream);
+    L.width = static_cast<int>(f->probe_width);
+    CF_CUDA(f->ops->remove(t, keys, n, out, L), "delete launch");
+    return CF_OK;
+}
+
 int cf_delete_async(cf_filter* f, const void* d_keys, uint64_t n, uint8_t* d_out, void* stream) {
     if (int s = check_batch(f, d_keys, n)) return s;
     f->known_empty = false;
@@ -806,17 +854,20 @@ int cf_delete_async(cf_filter* f, const void* d_keys, uint64_t n, uint8_t* d_out
     switch (choose_path(f, SEG_DELETE, n, false)) {
         case PATH_REGION: return run_region(f, SEG_DELETE, d_keys, n, d_out, stream);
         case PATH_SEGMENT: return run_segmented(f, SEG_DELETE, d_keys, n, d_out, stream);
-        default: break;
+        default: return do_delete(f, dev(f), d_keys, n, d_out, stream);
     }
-    LaunchCfg L = launch(f, KID_DELETE, stream);
-    L.width = static_cast<int>(f->probe_width);
-    CF_CUDA(f->ops->remove(dev(f), d_keys, n, d_out, L), "delete launch");
-    return CF_OK;
 }
 
 int cf_delete(cf_filter* f, const void* d_keys, uint64_t n, uint8_t* d_out, void* stream, uint64_t* occupied_out) {
-    if (int s = cf_delete_async(f, d_keys, n, d_out, stream)) return s;
+    if (int s = check_batch(f, d_keys, n)) return s;
     DeviceGuard g(f->device);
+    if (n && choose_path(f, SEG_DELETE, n, false) == PATH_RANDOM) {
+        f->known_empty = false;
+        const DevTable t = dev_published(f);
+        if (int s = do_delete(f, t, d_keys, n, d_out, stream)) return s;
+        return finish_published(t, stream, occupied_out);
+    }
+    if (int s = cf_delete_async(f, d_keys, n, d_out, stream)) return s;
     return finish(f, stream, occupied_out);
 }
 

@@ -51,6 +51,7 @@ enum Counter : int {
     CTR_HIST0 = 16,  // eviction-chain-length histogram, kChainBins counters
     CTR_COUNT = 32
 };
+constexpr int kPublished = 16;  // counters before the histogram
 // Chain-length bins: 0 evictions (a slot freed up), 1, 2-3, 4-7, ..., >= 256.
 constexpr int kChainBins = 10;
 constexpr uint64_t ERR_CAS_LIMIT = 1;   // a compare-and-swap retry bound was hit
@@ -61,6 +62,11 @@ struct DevTable {
     uint64_t nb_mask;
     unsigned long long* ctr;
     unsigned long long* hist = nullptr;  // chain-length histogram (kChainBins), or null when not recorded
+    // Host mirror (pinned) that the last CTA of a random insert or delete writes
+    // the first kPublished counters to, and the ticket that finds that CTA; null
+    // when the host reads them another way.
+    unsigned long long* pub = nullptr;
+    unsigned int* ticket = nullptr;
 };
 
 // Records the eviction chain of one stored key (L slot exchanges).
@@ -579,6 +585,26 @@ __device__ __forceinline__ void flush_counters(unsigned long long* ctr, const Co
     }
 }
 
+// After flush_counters: the last CTA of the grid to come here copies the counters
+// to the call's host mirror, so that a synchronous call needs no copy of its own
+// after the kernel (delete of 1000 keys, from Python: 20 us with one, 17.5 without).
+// Every thread of the CTA calls it.
+__device__ __forceinline__ void publish_counters(const DevTable& t) {
+    if (!t.pub) return;
+    __shared__ bool s_last;
+    if (threadIdx.x == 0) {
+        __threadfence();  // this CTA's counter updates come before its ticket (thread 0's warp made them)
+        s_last = atomicAdd(t.ticket, 1u) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!s_last) return;
+    if (threadIdx.x < kPublished) {
+        __threadfence();
+        t.pub[threadIdx.x] = *const_cast<volatile unsigned long long*>(&t.ctr[threadIdx.x]);
+    }
+    if (threadIdx.x == 0) *t.ticket = 0;
+}
+
 // ------------------------------------------------------------------ kernels
 
 template <class C, int KPT>
@@ -681,9 +707,13 @@ __global__ void __launch_bounds__(512) k_delete(DevTable t, const typename C::Ke
         removed += __popc(done);
         if (out) store_results<KPT>(out, k0, n, out_vec, done);
     }
+    if (__any_sync(0xFFFFFFFFu, err) && (threadIdx.x & 31) == 0) {
+        atomicOr(&t.ctr[CTR_ERROR], ERR_CAS_LIMIT);
+        __threadfence();
+    }
     const int32_t rem = static_cast<int32_t>(removed);
     flush_counters(t.ctr, {{CTR_REMOVED, rem}, {CTR_OCCUPIED, -rem}});
-    if (__any_sync(0xFFFFFFFFu, err) && (threadIdx.x & 31) == 0) atomicOr(&t.ctr[CTR_ERROR], ERR_CAS_LIMIT);
+    publish_counters(t);
 }
 
 // ------------------------------------------------- warp-cooperative probing
@@ -891,9 +921,13 @@ __global__ void __launch_bounds__(512) k_delete_coop(DevTable t, const typename 
             if (out && k0 < n) store_results<KPT>(out, k0, n, out_vec, done);
         }
     }
+    if (__any_sync(0xFFFFFFFFu, err) && (threadIdx.x & 31) == 0) {
+        atomicOr(&t.ctr[CTR_ERROR], ERR_CAS_LIMIT);
+        __threadfence();
+    }
     const int32_t rem = static_cast<int32_t>(removed);
     flush_counters(t.ctr, {{CTR_REMOVED, rem}, {CTR_OCCUPIED, -rem}});
-    if (__any_sync(0xFFFFFFFFu, err) && (threadIdx.x & 31) == 0) atomicOr(&t.ctr[CTR_ERROR], ERR_CAS_LIMIT);
+    publish_counters(t);
 }
 
 // Eviction for one key whose two buckets were full (CuckooFilter::insert,
@@ -1014,6 +1048,10 @@ __global__ void __launch_bounds__(512) k_insert(DevTable t, const typename C::Ke
         }
     }
     if (lane < pending) evict_parked(buf[lane]);
+    if (__any_sync(0xFFFFFFFFu, err) && (threadIdx.x & 31) == 0) {
+        atomicOr(&t.ctr[CTR_ERROR], ERR_CAS_LIMIT);
+        __threadfence();
+    }
     // a tag dropped by crossing eviction walks leaves the table one entry short
     flush_counters(t.ctr, {{CTR_OCCUPIED, static_cast<int32_t>(n_prim + n_sec + (n_evk - n_fail) - st.lost + st.dup)},
                            {CTR_DUP, static_cast<int32_t>(st.dup)},
@@ -1023,7 +1061,7 @@ __global__ void __launch_bounds__(512) k_insert(DevTable t, const typename C::Ke
                            {CTR_EVICTIONS, static_cast<int32_t>(st.evictions)},
                            {CTR_FAILED, static_cast<int32_t>(n_fail)},
                            {CTR_LOST, static_cast<int32_t>(st.lost)}});
-    if (__any_sync(0xFFFFFFFFu, err) && (threadIdx.x & 31) == 0) atomicOr(&t.ctr[CTR_ERROR], ERR_CAS_LIMIT);
+    publish_counters(t);
 }
 
 // Occupied-slot count of the whole table (countOccupiedSlots, CuckooFilter.cuh:759-785).

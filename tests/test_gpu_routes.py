@@ -256,3 +256,43 @@ def test_insertMany_route_by_batch_size(cfb, orc, n, load):
     f.clear()
     filled_and_emptied(cfb, f, [dev(keys)], False)
     f.close()
+
+
+@pytest.mark.parametrize("n", [1, 31, 512, 513, 40_000])
+def test_counts_of_synchronous_calls_from_several_threads(cfb, orc, n):
+    """The count a synchronous random insert or delete returns is written by its
+    own last CTA: threads that work on one filter at the same time, on streams of
+    their own, each get a count that lies between what was there before and after,
+    and the last ones agree with the table."""
+    import threading
+
+    cfg = cfb.CuckooConfig(T="uint64", bitsPerTag=16, bucketSize=16, evictionPolicy=cfb.EvictionPolicy.BFS)
+    f = cfb.CuckooFilter(cfg, 1 << 20)
+    rounds, nt = 6, 4
+    keys = [dev(orc.splitmix64(80 + i, n)) for i in range(nt)]
+    streams = [torch.cuda.Stream() for _ in range(nt)]
+    torch.cuda.synchronize()
+    bad = []
+
+    def work(i):
+        try:
+            with torch.cuda.stream(streams[i]):
+                for _ in range(rounds):
+                    a = f.insertMany(keys[i])
+                    b = f.deleteMany(keys[i])
+                    if not (n <= a <= nt * n and 0 <= b <= (nt - 1) * n):
+                        bad.append((i, a, b))
+        except Exception as e:  # noqa: BLE001
+            bad.append((i, repr(e)))
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(nt)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not bad, bad
+    assert f.occupiedSlots() == f.countOccupiedSlots() == 0
+    assert f.insertMany(keys[0]) == n == f.occupiedSlots()
+    assert f.insertMany(keys[0][:0]) == n and f.deleteMany(keys[0][:0]) == n  # nothing to launch
+    assert f.deleteMany(keys[0]) == 0
+    f.close()
