@@ -488,8 +488,16 @@ bool bin_geometry(const cf_filter* f, uint64_t m, BinGeom* g) {
 // been stored) when its workspace does not fit the limit or the batch is skewed.
 int run_binned(cf_filter* f, const void* keys, uint64_t n, uint8_t* out, void* stream, bool* taken) {
     *taken = false;
+    // A captured insert would replay what holds only now (an empty table, this
+    // workspace), so a capturing stream is left to the segment-staged path, whose
+    // host waits end the capture with an error.
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(static_cast<cudaStream_t>(stream), &capture) != cudaSuccess) {
+        cudaGetLastError();
+        return CF_OK;
+    }
     BinGeom g{};
-    if (!bin_geometry(f, n, &g)) return CF_OK;
+    if (capture != cudaStreamCaptureStatusNone || !bin_geometry(f, n, &g)) return CF_OK;
     auto al = [](uint64_t x) { return (x + 255) & ~255ull; };
     const uint64_t words = f->cfg.bucket_size <= 64 && g.sbl >= 5 ? (static_cast<uint64_t>(g.nseg) << g.sbl) >> 5 : 0;
     // a buffer holds first-pass bins in one round and segments' bins in another

@@ -296,3 +296,42 @@ def test_counts_of_synchronous_calls_from_several_threads(cfb, orc, n):
     assert f.insertMany(keys[0][:0]) == n and f.deleteMany(keys[0][:0]) == n  # nothing to launch
     assert f.deleteMany(keys[0]) == 0
     f.close()
+
+
+CAPTURE = """
+import __graft_entry__, oracle, torch
+cfb = __graft_entry__.package()
+cfg = cfb.CuckooConfig(T="uint64", bitsPerTag=16, bucketSize=16, evictionPolicy=cfb.EvictionPolicy.BFS)
+f = cfb.CuckooFilter(cfg, 1 << 18)
+keys = torch.from_numpy(oracle.splitmix64(91, int(0.9 * f.capacity())).view("int64")).cuda()
+n = keys.numel()
+f.insertMany(keys)  # the workspace exists
+f.clear()
+s = torch.cuda.Stream()
+s.wait_stream(torch.cuda.current_stream())
+refused = False
+try:
+    with torch.cuda.graph(torch.cuda.CUDAGraph(), stream=s):
+        f.insertManyAsync(keys, stream=s)
+except Exception:
+    refused = True
+torch.cuda.synchronize()
+try:
+    f.containsMany(keys)  # the CUDA runtime hands the refusal to the next call that asks for errors
+except cfb.CuckooError:
+    pass
+f.clear()
+assert refused and f.insertMany(keys) == n == f.countOccupiedSlots() and bool(f.containsMany(keys).all())
+print("refused, and the filter works on")
+"""
+
+
+def test_binned_insert_is_refused_under_capture(cfb, orc):
+    """A captured fill would replay with what was known of the table at capture
+    time, so it ends in an error, and the filter works on afterwards.  (In a
+    process of its own: a capture that fails leaves torch's allocator changed.)"""
+    import subprocess
+
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", CAPTURE], cwd=root, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and "works on" in r.stdout, r.stdout + r.stderr
