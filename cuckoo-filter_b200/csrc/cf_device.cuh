@@ -135,6 +135,16 @@ struct Cfg {
     using Key = typename std::conditional<KB == 8, uint64_t, uint32_t>::type;
 };
 
+// hb % n for a 32-bit hash and n >= 1: a 32-bit division (n past 32 bits leaves hb as it is).
+__host__ __device__ __forceinline__ uint64_t mod_hash32(uint32_t hb, uint64_t n) {
+    return (n >> 32) ? hb : hb % static_cast<uint32_t>(n);
+}
+
+// x % n for x < 2n: the sums and differences of two residues below.  (With a
+// 64-bit division each, the AddSub and Offset policies spent more instructions on
+// divisions than on the rest of a key; the one of the 64-bit hash remains.)
+__host__ __device__ __forceinline__ uint64_t mod_sum(uint64_t x, uint64_t n) { return x >= n ? x - n : x; }
+
 // Bucket derivation (getCandidateBuckets of the configured policy).
 // `nbm` is the bucket count minus one: the index mask of the XOR policy, whose
 // bucket count is a power of two; AddSub and Offset take any (even, for
@@ -147,12 +157,12 @@ __host__ __device__ __forceinline__ void candidates(uint64_t key, uint64_t nbm, 
         // (bitsPerTag - 1) fingerprint bits, choice bit 0 (:232-247)
         const uint32_t f = static_cast<uint32_t>(h >> 32) & (C::choice_bit - 1u);
         fp = f > 1u ? f : 1u;  // 0 -> 1, as a maximum
-        i1 = static_cast<uint64_t>(hb) % (nbm + 1);
+        i1 = mod_hash32(hb, nbm + 1);
     } else {
         const uint32_t f = static_cast<uint32_t>(h >> 32) & C::tag_mask;
         fp = f > 1u ? f : 1u;
         if constexpr (C::alt_policy == ALT_ADDSUB)
-            i1 = static_cast<uint64_t>(hb) % ((nbm + 1) / 2);  // first half (:128-137)
+            i1 = mod_hash32(hb, (nbm + 1) / 2);  // first half (:128-137)
         else
             i1 = static_cast<uint64_t>(hb) & nbm;
     }
@@ -165,13 +175,13 @@ __host__ __device__ __forceinline__ uint64_t alt_bucket(uint64_t b, uint32_t tag
         // first half -> second by adding, second -> first by subtracting (:150-160)
         const uint64_t half = (nbm + 1) / 2;
         const uint64_t fh = hash_tag<C::bits>(tag) % half;
-        return b < half ? ((b + fh) % half) + half : (b - fh) % half;
+        return b < half ? mod_sum(b + fh, half) + half : mod_sum(b - fh, half);
     } else if constexpr (C::alt_policy == ALT_OFFSET) {
         // +offset from the primary, -offset from the alternate (:300-323)
         const uint64_t nb = nbm + 1;
         uint64_t off = hash_tag<C::bits>(tag & (C::choice_bit - 1u)) % nb;
         off = off == 0 ? 1 : off;
-        return (tag & C::choice_bit) == 0 ? (b + off) % nb : (b + nb - off) % nb;
+        return (tag & C::choice_bit) == 0 ? mod_sum(b + off, nb) : mod_sum(b + nb - off, nb);
     } else {
         return b ^ (hash_tag<C::bits>(tag) & nbm);
     }
