@@ -20,8 +20,9 @@
 
 using namespace cfb;
 
-// Synchronous calls on one filter that may be in flight at a time (one host
-// thread each) before two share a row of published counters.
+// Rows of published counters of a filter.  A synchronous random insert or delete
+// holds one from before its launch until its stream has been waited for; a call
+// that finds none free reads the counters back with a copy instead.
 constexpr unsigned int kPubSlots = 64;
 
 struct cf_filter {
@@ -33,10 +34,11 @@ struct cf_filter {
     unsigned long long* d_ctr;  // CTR_COUNT device counters
     unsigned long long* h_ctr;  // pinned mirror
     // Counters as the last CTA of a synchronous random insert or delete leaves
-    // them: kPubSlots rows of kPublished, one per call in flight, and the rows' tickets.
+    // them: kPubSlots rows of kPublished, the rows' tickets (zero while a row is
+    // free) and one bit per free row.
     unsigned long long* h_pub;
     unsigned int* d_ticket;
-    std::atomic<unsigned int> pub_next;
+    std::atomic<uint64_t> pub_free;
     int device;
     int block;
     int max_grid[KID_COUNT_KERNELS];
@@ -213,23 +215,42 @@ int finish(cf_filter* f, void* stream, uint64_t* occupied_out) {
     return check_counters(f->h_ctr, occupied_out);
 }
 
-// The same after a random insert or delete launched with `t`, whose last CTA
-// wrote the counters to t.pub.
-int finish_published(const DevTable& t, void* stream, uint64_t* occupied_out) {
-    CF_CUDA(cudaStreamSynchronize(static_cast<cudaStream_t>(stream)), "stream synchronize");
-    unsigned long long c[kPublished];
-    for (int i = 0; i < kPublished; ++i) c[i] = static_cast<volatile unsigned long long*>(t.pub)[i];
-    return check_counters(c, occupied_out);
-}
-
-// The table with a row of published counters of this call's own.
-DevTable dev_published(cf_filter* f) {
-    DevTable t = dev(f);
-    const unsigned int slot = f->pub_next.fetch_add(1, std::memory_order_relaxed) % kPubSlots;
-    t.pub = f->h_pub + slot * kPublished;
-    t.ticket = f->d_ticket + slot;
-    return t;
-}
+// A row of published counters held by one synchronous call, or none when all are
+// in use.  It goes back only once the kernel that uses it has ended (which leaves
+// the ticket at zero): a call whose launch or wait failed keeps it from reuse.
+struct PubRow {
+    cf_filter* f;
+    int row = -1;
+    explicit PubRow(cf_filter* filter) : f(filter) {
+        uint64_t free = f->pub_free.load(std::memory_order_relaxed);
+        while (free) {
+            const int r = __builtin_ctzll(free);
+            if (f->pub_free.compare_exchange_weak(free, free & ~(1ull << r), std::memory_order_acquire)) {
+                row = r;
+                return;
+            }
+        }
+    }
+    DevTable table() const {
+        DevTable t = dev(f);
+        if (row >= 0) {
+            t.pub = f->h_pub + row * kPublished;
+            t.ticket = f->d_ticket + row;
+        }
+        return t;
+    }
+    // Waits for the random insert or delete launched with table(), whose last CTA
+    // has written the row.
+    int finish(void* stream, uint64_t* occupied_out) const {
+        if (row < 0) return ::finish(f, stream, occupied_out);
+        CF_CUDA(cudaStreamSynchronize(static_cast<cudaStream_t>(stream)), "stream synchronize");
+        unsigned long long c[kPublished];
+        const volatile unsigned long long* pub = f->h_pub + row * kPublished;
+        for (int i = 0; i < kPublished; ++i) c[i] = pub[i];
+        f->pub_free.fetch_or(1ull << row, std::memory_order_release);
+        return check_counters(c, occupied_out);
+    }
+};
 
 int ilog2(uint64_t v) { return 63 - __builtin_clzll(v); }
 
@@ -743,6 +764,8 @@ int cf_create(const cf_config* cfg, uint64_t capacity, cf_filter** out) {
     if (e == cudaSuccess)
         e = cudaHostAlloc(&f->h_ctr, (CTR_COUNT + kPubSlots * kPublished) * sizeof(unsigned long long), cudaHostAllocDefault);
     if (e == cudaSuccess) f->h_pub = f->h_ctr + CTR_COUNT;
+    static_assert(kPubSlots == 64, "one bit of pub_free per row");
+    f->pub_free = ~0ull;
     if (e == cudaSuccess) e = cudaMemset(f->d_table, 0, f->table_bytes);
     if (e == cudaSuccess) e = cudaMemset(f->d_ctr, 0, kCtrBytes);
     if (e == cudaSuccess) e = cudaDeviceSynchronize();
@@ -808,9 +831,9 @@ int cf_insert(cf_filter* f, const void* d_keys, uint64_t n, uint8_t* d_out, void
     if (int s = check_batch(f, d_keys, n)) return s;
     DeviceGuard g(f->device);
     if (n && choose_path(f, SEG_INSERT, n, false) == PATH_RANDOM) {
-        const DevTable t = dev_published(f);
-        if (int s = do_insert(f, t, d_keys, n, d_out, stream)) return s;
-        return finish_published(t, stream, occupied_out);
+        const PubRow row(f);
+        if (int s = do_insert(f, row.table(), d_keys, n, d_out, stream)) return s;
+        return row.finish(stream, occupied_out);
     }
     if (int s = insert_any(f, d_keys, n, d_out, stream, false)) return s;
     return finish(f, stream, occupied_out);
@@ -871,9 +894,9 @@ int cf_delete(cf_filter* f, const void* d_keys, uint64_t n, uint8_t* d_out, void
     DeviceGuard g(f->device);
     if (n && choose_path(f, SEG_DELETE, n, false) == PATH_RANDOM) {
         f->known_empty = false;
-        const DevTable t = dev_published(f);
-        if (int s = do_delete(f, t, d_keys, n, d_out, stream)) return s;
-        return finish_published(t, stream, occupied_out);
+        const PubRow row(f);
+        if (int s = do_delete(f, row.table(), d_keys, n, d_out, stream)) return s;
+        return row.finish(stream, occupied_out);
     }
     if (int s = cf_delete_async(f, d_keys, n, d_out, stream)) return s;
     return finish(f, stream, occupied_out);

@@ -298,6 +298,82 @@ def test_counts_of_synchronous_calls_from_several_threads(cfb, orc, n):
     f.close()
 
 
+def test_counts_while_a_long_call_is_in_flight(cfb, orc):
+    """One thread makes hundreds of small synchronous calls on a high-priority
+    stream while another's large deletes run (of keys that are not there): every
+    count is the call's own, and none is stale afterwards."""
+    import threading
+
+    cfg = cfb.CuckooConfig(T="uint64", bitsPerTag=32, bucketSize=8, evictionPolicy=cfb.EvictionPolicy.BFS)
+    f = cfb.CuckooFilter(cfg, 1 << 28)
+    absent = dev(orc.splitmix64(101, 1 << 24)).repeat(8)
+    small = dev(orc.splitmix64(102, 1000))
+    torch.cuda.synchronize()
+    bad, done, long_counts = [], threading.Event(), []
+
+    def long_calls():
+        try:
+            with torch.cuda.stream(torch.cuda.Stream()):
+                for _ in range(8):
+                    long_counts.append(f.deleteMany(absent))
+        except Exception as e:  # noqa: BLE001
+            bad.append(repr(e))
+        done.set()
+
+    t = threading.Thread(target=long_calls)
+    t.start()
+    stored = 0
+    with torch.cuda.stream(torch.cuda.Stream(priority=-1)):
+        while (not done.is_set() or stored < 300) and stored < 800:
+            got = f.insertMany(small[stored:stored + 1])
+            stored += 1
+            if got != stored:
+                bad.append((stored, got))
+    t.join()
+    for _ in range(130):
+        got = f.insertMany(small[stored:stored + 1])
+        stored += 1
+        if got != stored:
+            bad.append((stored, got))
+    assert not bad, bad[:5]
+    assert len(long_counts) == 8 and long_counts == sorted(long_counts) and 0 <= long_counts[0] <= long_counts[-1] <= stored
+    assert f.occupiedSlots() == f.countOccupiedSlots() == stored
+    f.close()
+
+
+def test_counts_of_more_calls_than_rows(cfb, orc):
+    """More threads than a filter has rows of published counters."""
+    import threading
+
+    cfg = cfb.CuckooConfig(T="uint64", bitsPerTag=16, bucketSize=16, evictionPolicy=cfb.EvictionPolicy.BFS)
+    f = cfb.CuckooFilter(cfg, 1 << 20)
+    n, rounds, nt = 513, 4, 80
+    keys = [dev(orc.splitmix64(200 + i, n)) for i in range(nt)]
+    streams = [torch.cuda.Stream() for _ in range(nt)]
+    torch.cuda.synchronize()
+    bad = []
+
+    def work(i):
+        try:
+            for _ in range(rounds):
+                a = f.insertMany(keys[i], stream=streams[i])
+                b = f.deleteMany(keys[i], stream=streams[i])
+                if not (n <= a <= nt * n and 0 <= b <= (nt - 1) * n):
+                    bad.append((i, a, b))
+        except Exception as e:  # noqa: BLE001
+            bad.append((i, repr(e)))
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(nt)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not bad, bad[:5]
+    for k in range(130):
+        assert f.insertMany(keys[k % nt][k:k + 1]) == k + 1
+    f.close()
+
+
 CAPTURE = """
 import __graft_entry__, oracle, torch
 cfb = __graft_entry__.package()
