@@ -13,6 +13,7 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <mutex>
 #include <vector>
 
 #include "../../include/cuckoo_b200.h"
@@ -65,8 +66,17 @@ struct cf_filter {
     // The table is all zeros (set by cf_create and cf_clear, which synchronize;
     // cleared by every call that may write the table).  Never set again once
     // cf_table has handed out the table's address (table_exposed).
-    bool known_empty;
+    std::atomic<bool> known_empty;
     bool table_exposed;
+    // Staged batches (segment-staged, binned, region-staged) of a filter share its
+    // workspace and write whole segments of the table back, so they run one after
+    // the other whatever their streams: staged_mu is held while one is enqueued
+    // (until it has ended, in a synchronous call), and staged_ev marks the end of the
+    // last asynchronous one, on the stream with id staged_stream, while staged_pending.
+    std::mutex staged_mu;
+    cudaEvent_t staged_ev;
+    unsigned long long staged_stream;
+    std::atomic<bool> staged_pending;
     uint32_t persistent;    // CF_OPT_PERSISTENT (0 = one tile per CTA, 1 = persistent grid)
     uint32_t chain_hist;    // CF_OPT_CHAIN_HISTOGRAM
 };
@@ -251,6 +261,67 @@ struct PubRow {
         return check_counters(c, occupied_out);
     }
 };
+
+// A capturing stream, or one that cannot be asked (another stream's capture forbids it).
+bool is_capturing(cudaStream_t s) {
+    cudaStreamCaptureStatus c = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &c) == cudaSuccess) return c != cudaStreamCaptureStatusNone;
+    cudaGetLastError();
+    return true;
+}
+
+// Work enqueued on `stream` from here on follows the last asynchronous staged
+// batch.  Not under capture: an event from outside cannot be waited for there, and
+// the graph's launches are ordered by whoever launches it.  Holds staged_mu.
+int follow_staged_locked(cf_filter* f, void* stream) {
+    if (!f->staged_pending) return CF_OK;
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    unsigned long long id = 0;  // of the stream itself: a handle can be used again for another
+    if (cudaStreamGetId(s, &id) == cudaSuccess) {
+        if (id == f->staged_stream) return CF_OK;
+    } else {
+        cudaGetLastError();
+    }
+    if (is_capturing(s)) return CF_OK;
+    CF_CUDA(cudaStreamWaitEvent(s, f->staged_ev, 0), "wait for the batch before");
+    return CF_OK;
+}
+
+// The same for a call that is not a staged batch itself.
+int follow_staged(cf_filter* f, void* stream) {
+    if (!f->staged_pending.load(std::memory_order_acquire)) return CF_OK;
+    std::lock_guard<std::mutex> lock(f->staged_mu);
+    return follow_staged_locked(f, stream);
+}
+
+// Marks the end of an asynchronous staged batch.
+int note_staged_locked(cf_filter* f, void* stream) {
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    if (is_capturing(s)) return CF_OK;
+    CF_CUDA(cudaStreamGetId(s, &f->staged_stream), "stream id");
+    CF_CUDA(cudaEventRecord(f->staged_ev, s), "mark the end of the batch");
+    f->staged_pending.store(true, std::memory_order_release);
+    return CF_OK;
+}
+
+// A staged batch: run() enqueues it; with `wait` the call returns when it has
+// ended, with the occupied count.
+template <class Run>
+int staged_batch(cf_filter* f, void* stream, bool wait, uint64_t* occupied_out, Run run) {
+    std::lock_guard<std::mutex> lock(f->staged_mu);
+    if (int st = follow_staged_locked(f, stream)) return st;
+    int st = run();
+    if (wait && st == CF_OK) {
+        st = finish(f, stream, occupied_out);
+        if (st == CF_OK) {
+            f->staged_pending.store(false, std::memory_order_release);
+            return CF_OK;
+        }
+    }
+    // (an error may have left part of the batch in flight)
+    const int noted = note_staged_locked(f, stream);
+    return st ? st : noted;
+}
 
 int ilog2(uint64_t v) { return 63 - __builtin_clzll(v); }
 
@@ -512,13 +583,8 @@ int run_binned(cf_filter* f, const void* keys, uint64_t n, uint8_t* out, void* s
     // A captured insert would replay what holds only now (an empty table, this
     // workspace), so a capturing stream is left to the segment-staged path, whose
     // host waits end the capture with an error.
-    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(static_cast<cudaStream_t>(stream), &capture) != cudaSuccess) {
-        cudaGetLastError();
-        return CF_OK;
-    }
     BinGeom g{};
-    if (capture != cudaStreamCaptureStatusNone || !bin_geometry(f, n, &g)) return CF_OK;
+    if (is_capturing(static_cast<cudaStream_t>(stream)) || !bin_geometry(f, n, &g)) return CF_OK;
     auto al = [](uint64_t x) { return (x + 255) & ~255ull; };
     const uint64_t words = f->cfg.bucket_size <= 64 && g.sbl >= 5 ? (static_cast<uint64_t>(g.nseg) << g.sbl) >> 5 : 0;
     // a buffer holds first-pass bins in one round and segments' bins in another
@@ -766,6 +832,7 @@ int cf_create(const cf_config* cfg, uint64_t capacity, cf_filter** out) {
     if (e == cudaSuccess) f->h_pub = f->h_ctr + CTR_COUNT;
     static_assert(kPubSlots == 64, "one bit of pub_free per row");
     f->pub_free = ~0ull;
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&f->staged_ev, cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaMemset(f->d_table, 0, f->table_bytes);
     if (e == cudaSuccess) e = cudaMemset(f->d_ctr, 0, kCtrBytes);
     if (e == cudaSuccess) e = cudaDeviceSynchronize();
@@ -787,6 +854,7 @@ int cf_destroy(cf_filter* f) {
     if (f->h_ctr) cudaFreeHost(f->h_ctr);
     if (f->h_cnt) cudaFreeHost(f->h_cnt);
     if (f->ws) cudaFree(f->ws);
+    if (f->staged_ev) cudaEventDestroy(f->staged_ev);
     delete f;
     return CF_OK;
 }
@@ -802,41 +870,46 @@ int cf_get_info(const cf_filter* f, cf_info* out) {
     return CF_OK;
 }
 
-int insert_any(cf_filter* f, const void* keys, uint64_t n, uint8_t* out, void* stream, bool sorted) {
+// Enqueues an insert; with `wait` it returns when the insert has ended, with the occupied count.
+int insert_any(cf_filter* f, const void* keys, uint64_t n, uint8_t* out, void* stream, bool sorted, bool wait,
+               uint64_t* occupied_out) {
     switch (choose_path(f, SEG_INSERT, n, sorted)) {
-        case PATH_REGION: return run_region(f, SEG_INSERT, keys, n, out, stream);
-        case PATH_SEGMENT: {
-            // At least one key per bucket: slot order within a bucket is
-            // unspecified, and the batch is binned (fills to 0.95, segment-staged
-            // against binned: 2^20 slots 420 -> 198 us, 2^28 6.58 -> 4.75 ms with a
-            // sample looked up, 2^31 45.8 -> 36.5 ms).  Buckets of more than 16
-            // slots, batches that do not fit the workspace limit in one piece and
-            // skewed ones with a short list stay segment-staged.
-            bool taken = false;
-            if (n >= f->num_buckets)
-                if (int st = run_binned(f, keys, n, out, stream, &taken)) return st;
-            return taken ? CF_OK : run_segmented(f, SEG_INSERT, keys, n, out, stream);
-        }
-        default: return do_insert(f, dev(f), keys, n, out, stream);
+        case PATH_REGION:
+            return staged_batch(f, stream, wait, occupied_out,
+                                [&] { return run_region(f, SEG_INSERT, keys, n, out, stream); });
+        case PATH_SEGMENT:
+            return staged_batch(f, stream, wait, occupied_out, [&]() -> int {
+                // At least one key per bucket: slot order within a bucket is
+                // unspecified, and the batch is binned (fills to 0.95, segment-staged
+                // against binned: 2^20 slots 420 -> 198 us, 2^28 6.58 -> 4.75 ms with a
+                // sample looked up, 2^31 45.8 -> 36.5 ms).  Buckets of more than 16
+                // slots, batches that do not fit the workspace limit in one piece and
+                // skewed ones with a short list stay segment-staged.
+                bool taken = false;
+                if (n >= f->num_buckets)
+                    if (int st = run_binned(f, keys, n, out, stream, &taken)) return st;
+                return taken ? CF_OK : run_segmented(f, SEG_INSERT, keys, n, out, stream);
+            });
+        default: break;
     }
+    if (int s = follow_staged(f, stream)) return s;
+    if (!wait) return do_insert(f, dev(f), keys, n, out, stream);
+    if (!n) return finish(f, stream, occupied_out);
+    const PubRow row(f);
+    if (int s = do_insert(f, row.table(), keys, n, out, stream)) return s;
+    return row.finish(stream, occupied_out);
 }
 
 int cf_insert_async(cf_filter* f, const void* d_keys, uint64_t n, uint8_t* d_out, void* stream) {
     if (int s = check_batch(f, d_keys, n)) return s;
     DeviceGuard g(f->device);
-    return insert_any(f, d_keys, n, d_out, stream, false);
+    return insert_any(f, d_keys, n, d_out, stream, false, false, nullptr);
 }
 
 int cf_insert(cf_filter* f, const void* d_keys, uint64_t n, uint8_t* d_out, void* stream, uint64_t* occupied_out) {
     if (int s = check_batch(f, d_keys, n)) return s;
     DeviceGuard g(f->device);
-    if (n && choose_path(f, SEG_INSERT, n, false) == PATH_RANDOM) {
-        const PubRow row(f);
-        if (int s = do_insert(f, row.table(), d_keys, n, d_out, stream)) return s;
-        return row.finish(stream, occupied_out);
-    }
-    if (int s = insert_any(f, d_keys, n, d_out, stream, false)) return s;
-    return finish(f, stream, occupied_out);
+    return insert_any(f, d_keys, n, d_out, stream, false, true, occupied_out);
 }
 
 int cf_insert_sorted(cf_filter* f, const void* d_keys, uint64_t n, uint8_t* d_out, void* stream,
@@ -844,8 +917,7 @@ int cf_insert_sorted(cf_filter* f, const void* d_keys, uint64_t n, uint8_t* d_ou
     if (int s = check_batch(f, d_keys, n)) return s;
     DeviceGuard g(f->device);
     // (bucket << bits) | tag must fit 64 bits for the staged paths; else the plain path
-    if (int s = insert_any(f, d_keys, n, d_out, stream, true)) return s;
-    return finish(f, stream, occupied_out);
+    return insert_any(f, d_keys, n, d_out, stream, true, true, occupied_out);
 }
 
 int cf_contains_async(cf_filter* f, const void* d_keys, uint64_t n, uint8_t* d_out, void* stream) {
@@ -853,10 +925,15 @@ int cf_contains_async(cf_filter* f, const void* d_keys, uint64_t n, uint8_t* d_o
     if (n && !d_out) return fail(CF_ERR_INVALID, "d_out is NULL with n > 0");
     DeviceGuard g(f->device);
     switch (choose_path(f, SEG_CONTAINS, n, false)) {
-        case PATH_REGION: return run_region(f, SEG_CONTAINS, d_keys, n, d_out, stream);
-        case PATH_SEGMENT: return run_segmented(f, SEG_CONTAINS, d_keys, n, d_out, stream);
+        case PATH_REGION:
+            return staged_batch(f, stream, false, nullptr,
+                                [&] { return run_region(f, SEG_CONTAINS, d_keys, n, d_out, stream); });
+        case PATH_SEGMENT:
+            return staged_batch(f, stream, false, nullptr,
+                                [&] { return run_segmented(f, SEG_CONTAINS, d_keys, n, d_out, stream); });
         default: break;
     }
+    if (int s = follow_staged(f, stream)) return s;
     LaunchCfg L = launch(f, KID_CONTAINS, stream);
     L.kpt = static_cast<int>(f->lookup_kpt);
     L.width = static_cast<int>(f->probe_width);
@@ -878,33 +955,42 @@ int do_delete(cf_filter* f, const DevTable& t, const void* keys, uint64_t n, uin
     return CF_OK;
 }
 
+// Enqueues a delete; with `wait` it returns when the delete has ended, with the occupied count.
+int delete_any(cf_filter* f, const void* keys, uint64_t n, uint8_t* out, void* stream, bool wait, uint64_t* occupied_out) {
+    f->known_empty = false;
+    switch (choose_path(f, SEG_DELETE, n, false)) {
+        case PATH_REGION:
+            return staged_batch(f, stream, wait, occupied_out,
+                                [&] { return run_region(f, SEG_DELETE, keys, n, out, stream); });
+        case PATH_SEGMENT:
+            return staged_batch(f, stream, wait, occupied_out,
+                                [&] { return run_segmented(f, SEG_DELETE, keys, n, out, stream); });
+        default: break;
+    }
+    if (int s = follow_staged(f, stream)) return s;
+    if (!wait) return do_delete(f, dev(f), keys, n, out, stream);
+    if (!n) return finish(f, stream, occupied_out);
+    const PubRow row(f);
+    if (int s = do_delete(f, row.table(), keys, n, out, stream)) return s;
+    return row.finish(stream, occupied_out);
+}
+
 int cf_delete_async(cf_filter* f, const void* d_keys, uint64_t n, uint8_t* d_out, void* stream) {
     if (int s = check_batch(f, d_keys, n)) return s;
-    f->known_empty = false;
     DeviceGuard g(f->device);
-    switch (choose_path(f, SEG_DELETE, n, false)) {
-        case PATH_REGION: return run_region(f, SEG_DELETE, d_keys, n, d_out, stream);
-        case PATH_SEGMENT: return run_segmented(f, SEG_DELETE, d_keys, n, d_out, stream);
-        default: return do_delete(f, dev(f), d_keys, n, d_out, stream);
-    }
+    return delete_any(f, d_keys, n, d_out, stream, false, nullptr);
 }
 
 int cf_delete(cf_filter* f, const void* d_keys, uint64_t n, uint8_t* d_out, void* stream, uint64_t* occupied_out) {
     if (int s = check_batch(f, d_keys, n)) return s;
     DeviceGuard g(f->device);
-    if (n && choose_path(f, SEG_DELETE, n, false) == PATH_RANDOM) {
-        f->known_empty = false;
-        const PubRow row(f);
-        if (int s = do_delete(f, row.table(), d_keys, n, d_out, stream)) return s;
-        return row.finish(stream, occupied_out);
-    }
-    if (int s = cf_delete_async(f, d_keys, n, d_out, stream)) return s;
-    return finish(f, stream, occupied_out);
+    return delete_any(f, d_keys, n, d_out, stream, true, occupied_out);
 }
 
 int cf_clear(cf_filter* f, void* stream) {
     if (int s = check_filter(f)) return s;
     DeviceGuard g(f->device);
+    if (int st = follow_staged(f, stream)) return st;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     CF_CUDA(cudaMemsetAsync(f->d_table, 0, f->table_bytes, s), "table clear");
     CF_CUDA(cudaMemsetAsync(f->d_ctr, 0, CTR_COUNT * sizeof(unsigned long long), s), "counter clear");
@@ -993,6 +1079,7 @@ int cf_load_table(cf_filter* f, const void* src, uint64_t bytes, void* stream) {
                     static_cast<unsigned long long>(f->table_bytes));
     DeviceGuard g(f->device);
     f->known_empty = false;
+    if (int st = follow_staged(f, stream)) return st;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     CF_CUDA(cudaMemcpyAsync(f->d_table, src, bytes, cudaMemcpyDefault, s), "table load");
     CF_CUDA(cudaMemsetAsync(f->d_ctr + CTR_OCCUPIED, 0, sizeof(unsigned long long), s), "counter reset");
@@ -1085,6 +1172,7 @@ int cf_store_table(cf_filter* f, void* dst, uint64_t bytes, void* stream) {
         return fail(CF_ERR_INVALID, "buffer is %llu bytes, table is %llu", static_cast<unsigned long long>(bytes),
                     static_cast<unsigned long long>(f->table_bytes));
     DeviceGuard g(f->device);
+    if (int st = follow_staged(f, stream)) return st;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     CF_CUDA(cudaMemcpyAsync(dst, f->d_table, bytes, cudaMemcpyDefault, s), "table store");
     CF_CUDA(cudaStreamSynchronize(s), "stream synchronize");
@@ -1161,6 +1249,7 @@ int cf_probe_count(cf_filter* f, const void* d_keys, uint64_t n, uint64_t* prima
     if (int s = check_batch(f, d_keys, n)) return s;
     if (!primary_hits) return fail(CF_ERR_INVALID, "primary_hits is NULL");
     DeviceGuard g(f->device);
+    if (int st = follow_staged(f, stream)) return st;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     unsigned long long* d_res = nullptr;
     CF_CUDA(cudaMalloc(&d_res, sizeof(unsigned long long)), "scratch allocation");
@@ -1273,14 +1362,15 @@ int cf_insert_sorted_noalloc(cf_filter* f, const void* d_keys, uint64_t n, uint8
     w.rg_grid = f->sms * 4;
     w.round2_segmented_min = f->round2_min ? f->round2_min : auto_threshold(f, SEG_INSERT);
     w.round1_cap = f->round1_cap;
-    if (n) {
+    return staged_batch(f, stream, true, occupied_out, [&]() -> int {
         // the segment pass clears the list counters, the result bitmap and the
         // segment starts itself; the other buffers are written before read
-        CF_CUDA(f->ops->seg_chunk(dev(f), f->geom, w, SEG_INSERT, d_keys, n, d_out, static_cast<cudaStream_t>(stream),
-                                  f->cfg.eviction_policy == CF_EVICT_BFS ? 1u : 0u, f->cfg.max_evictions),
-                "segment-staged batch");
-    }
-    return finish(f, stream, occupied_out);
+        if (n)
+            CF_CUDA(f->ops->seg_chunk(dev(f), f->geom, w, SEG_INSERT, d_keys, n, d_out, static_cast<cudaStream_t>(stream),
+                                      f->cfg.eviction_policy == CF_EVICT_BFS ? 1u : 0u, f->cfg.max_evictions),
+                    "segment-staged batch");
+        return CF_OK;
+    });
 }
 
 }  // extern "C"

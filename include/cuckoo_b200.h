@@ -160,7 +160,17 @@ int cf_delete(cf_filter* f, const void* d_keys, uint64_t n, uint8_t* d_out, void
               uint64_t* occupied_out);
 
 /* Asynchronous forms: enqueue on `stream` and return; counters stay on the
- * device (read them with cf_occupied / cf_get_stats, which synchronize). */
+ * device (read them with cf_occupied / cf_get_stats, which synchronize).  The
+ * keys and the results must stay allocated until the stream has passed the call.
+ *
+ * Streams and threads: calls on one filter may come from several threads and go
+ * to several streams.  Batches that probe at random may overlap.  Staged batches
+ * (CF_OPT_SEGMENTED_MIN_KEYS) share the filter's workspace and write whole segments
+ * of the table back: one starts on the device when the last one has ended, and
+ * every later call follows an asynchronous one, whatever their streams.  What the
+ * caller still has to order is a staged batch after another stream's random
+ * inserts and deletes that may be running (an event, or a synchronous call), and the
+ * launches of captured graphs. */
 int cf_insert_async(cf_filter* f, const void* d_keys, uint64_t n, uint8_t* d_out, void* stream);
 int cf_contains_async(cf_filter* f, const void* d_keys, uint64_t n, uint8_t* d_out, void* stream);
 int cf_delete_async(cf_filter* f, const void* d_keys, uint64_t n, uint8_t* d_out, void* stream);

@@ -374,6 +374,87 @@ def test_counts_of_more_calls_than_rows(cfb, orc):
     f.close()
 
 
+@pytest.mark.parametrize("staging", ["auto", "segment", "region"])
+@pytest.mark.parametrize("results", [False, True])
+def test_staged_batches_on_two_streams(cfb, orc, staging, results):
+    """Asynchronous staged batches of one filter on several streams, with nothing
+    between them: they share one workspace and the table, and leave what they
+    would leave one after the other.  So do calls that follow one on another stream."""
+    cfg = cfb.CuckooConfig(T="uint64", bitsPerTag=16, bucketSize=16, evictionPolicy=cfb.EvictionPolicy.BFS)
+    f = cfb.CuckooFilter(cfg, 1 << 24)
+    f.setOption(cfb.OPT_STAGING, {"auto": cfb.STAGING_AUTO, "segment": cfb.STAGING_SEGMENT, "region": cfb.STAGING_REGION}[staging])
+    n = 5 << 20
+    a, b, few = dev(orc.splitmix64(301, n)), dev(orc.splitmix64(302, n + 77)), dev(orc.splitmix64(303, 1000))
+    oks = [torch.full((k.numel(),), 7, dtype=torch.uint8, device="cuda") if results else None for k in (a, b, few)]
+    s1, s2, s3 = (torch.cuda.Stream() for _ in range(3))
+    for _ in range(3):
+        f.clear()
+        torch.cuda.synchronize()
+        f.insertManyAsync(a, stream=s1, d_output=oks[0])
+        f.insertManyAsync(b, stream=s2, d_output=oks[1])
+        f.insertManyAsync(few, stream=s3, d_output=oks[2])  # (at random, left to itself)
+        f.deleteManyAsync(few, stream=s3)
+        torch.cuda.synchronize()
+        assert f.occupiedSlots() == f.countOccupiedSlots() == a.numel() + b.numel()
+        st = f.stats()
+        assert st["failed"] == st["lost"] == st["duplicates"] == 0 and st["removed"] == 1000
+        assert bool(f.containsMany(a).all()) and bool(f.containsMany(b).all())
+        for k, ok in zip((a, b, few), oks):
+            assert ok is None or int(ok.sum()) == k.numel()
+        f.insertManyAsync(few, stream=s2)
+        f.deleteManyAsync(b, stream=s3)
+        f.deleteManyAsync(a, stream=s1)
+        torch.cuda.synchronize()
+        assert f.occupiedSlots() == f.countOccupiedSlots() == 1000
+        f.insertManyAsync(a, stream=s1)
+        f.clear(stream=s2)
+        torch.cuda.synchronize()
+        assert f.occupiedSlots() == f.countOccupiedSlots() == 0
+    f.close()
+
+
+def test_staged_batches_of_several_threads(cfb, orc):
+    """Threads that insert and delete staged batches of one filter at the same time, the
+    workspace growing between them; every count lies between what other threads can leave."""
+    import threading
+
+    cfg = cfb.CuckooConfig(T="uint64", bitsPerTag=16, bucketSize=16, evictionPolicy=cfb.EvictionPolicy.BFS)
+    f = cfb.CuckooFilter(cfg, 1 << 23)
+    sizes = [1 << 20, (1 << 20) + 5, 3 << 19, 7 << 18]
+    keys = [dev(orc.splitmix64(310 + i, n)) for i, n in enumerate(sizes)]
+    streams = [torch.cuda.Stream() for _ in sizes]
+    f.setOption(cfb.OPT_SEGMENTED_MIN_KEYS, 1)  # deletes too
+    torch.cuda.synchronize()
+    bad = []
+
+    def work(i):
+        try:
+            for r in range(4):
+                a = f.insertMany(keys[i], stream=streams[i])
+                if r & 1:
+                    f.deleteManyAsync(keys[i], stream=streams[i])
+                    b = 0
+                else:
+                    b = f.deleteMany(keys[i], stream=streams[i])
+                if not (sizes[i] <= a <= sum(sizes) and 0 <= b <= sum(sizes) - sizes[i]):
+                    bad.append((i, a, b))
+        except Exception as e:  # noqa: BLE001
+            bad.append((i, repr(e)))
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(len(sizes))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    torch.cuda.synchronize()
+    assert not bad, bad[:5]
+    st = f.stats()
+    assert st["failed"] == st["lost"] == st["duplicates"] == 0
+    assert f.occupiedSlots() == f.countOccupiedSlots() == 0
+    assert f.insertMany(keys[0]) == sizes[0] and bool(f.containsMany(keys[0]).all())
+    f.close()
+
+
 CAPTURE = """
 import __graft_entry__, oracle, torch
 cfb = __graft_entry__.package()
