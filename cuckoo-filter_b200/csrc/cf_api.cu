@@ -294,6 +294,10 @@ int follow_staged(cf_filter* f, void* stream) {
     return follow_staged_locked(f, stream);
 }
 
+// The same for the blocking reads and writes of the counters, which go to the
+// legacy default stream (non-blocking streams do not order themselves with it).
+int follow_staged(cf_filter* f) { return follow_staged(f, nullptr); }
+
 // Marks the end of an asynchronous staged batch.
 int note_staged_locked(cf_filter* f, void* stream) {
     cudaStream_t s = static_cast<cudaStream_t>(stream);
@@ -1003,6 +1007,7 @@ int cf_occupied(cf_filter* f, uint64_t* out) {
     if (int s = check_filter(f)) return s;
     if (!out) return fail(CF_ERR_INVALID, "out is NULL");
     DeviceGuard g(f->device);
+    if (int s = follow_staged(f)) return s;
     unsigned long long v = 0;
     CF_CUDA(cudaMemcpy(&v, f->d_ctr + CTR_OCCUPIED, sizeof(v), cudaMemcpyDeviceToHost), "occupancy read");
     *out = v;
@@ -1013,6 +1018,7 @@ int cf_count_occupied_slots(cf_filter* f, uint64_t* out) {
     if (int s = check_filter(f)) return s;
     if (!out) return fail(CF_ERR_INVALID, "out is NULL");
     DeviceGuard g(f->device);
+    if (int s = follow_staged(f)) return s;
     unsigned long long* d_res = nullptr;
     CF_CUDA(cudaMalloc(&d_res, sizeof(unsigned long long)), "scratch allocation");
     unsigned long long v = 0;
@@ -1029,6 +1035,7 @@ int cf_get_stats(cf_filter* f, cf_stats* out) {
     if (int s = check_filter(f)) return s;
     if (!out) return fail(CF_ERR_INVALID, "out is NULL");
     DeviceGuard g(f->device);
+    if (int s = follow_staged(f)) return s;
     unsigned long long c[CTR_COUNT];
     CF_CUDA(cudaMemcpy(c, f->d_ctr, sizeof(c), cudaMemcpyDeviceToHost), "counter read");
     out->occupied = c[CTR_OCCUPIED];
@@ -1047,6 +1054,7 @@ int cf_get_chain_histogram(cf_filter* f, uint64_t* bins) {
     if (int s = check_filter(f)) return s;
     if (!bins) return fail(CF_ERR_INVALID, "bins is NULL");
     DeviceGuard g(f->device);
+    if (int s = follow_staged(f)) return s;
     unsigned long long h[kChainBins];
     CF_CUDA(cudaMemcpy(h, f->d_ctr + CTR_HIST0, sizeof(h), cudaMemcpyDeviceToHost), "histogram read");
     for (int i = 0; i < kChainBins; ++i) bins[i] = h[i];
@@ -1056,6 +1064,7 @@ int cf_get_chain_histogram(cf_filter* f, uint64_t* bins) {
 int cf_reset_stats(cf_filter* f) {
     if (int s = check_filter(f)) return s;
     DeviceGuard g(f->device);
+    if (int s = follow_staged(f)) return s;
     CF_CUDA(cudaMemset(f->d_ctr + 1, 0, (CTR_COUNT - 1) * sizeof(unsigned long long)), "counter reset");
     return CF_OK;
 }

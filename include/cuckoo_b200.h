@@ -160,7 +160,8 @@ int cf_delete(cf_filter* f, const void* d_keys, uint64_t n, uint8_t* d_out, void
               uint64_t* occupied_out);
 
 /* Asynchronous forms: enqueue on `stream` and return; counters stay on the
- * device (read them with cf_occupied / cf_get_stats, which synchronize).  The
+ * device (read them with cf_occupied / cf_get_stats, which wait for staged batches
+ * and for blocking streams; synchronize a non-blocking stream yourself).  The
  * keys and the results must stay allocated until the stream has passed the call.
  *
  * Streams and threads: calls on one filter may come from several threads and go
@@ -178,7 +179,7 @@ int cf_delete_async(cf_filter* f, const void* d_keys, uint64_t n, uint8_t* d_out
 /* void clear() (CuckooFilter.cuh:675-682): zero the table and the counters. */
 int cf_clear(cf_filter* f, void* stream);
 
-/* size_t occupiedSlots() (CuckooFilter.cuh:699-704). Synchronizes the device. */
+/* size_t occupiedSlots() (CuckooFilter.cuh:699-704). Waits as described above. */
 int cf_occupied(cf_filter* f, uint64_t* out);
 
 /* size_t countOccupiedSlots() (CuckooFilter.cuh:759-785): counts non-empty

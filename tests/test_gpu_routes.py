@@ -413,6 +413,31 @@ def test_staged_batches_on_two_streams(cfb, orc, staging, results):
     f.close()
 
 
+def test_counters_read_after_an_asynchronous_staged_batch(cfb, orc):
+    """Every read of the counters waits for the staged batch before it, on a stream
+    that the legacy default stream does not wait for by itself."""
+    cfg = cfb.CuckooConfig(T="uint64", bitsPerTag=16, bucketSize=16, evictionPolicy=cfb.EvictionPolicy.BFS)
+    f = cfb.CuckooFilter(cfg, 1 << 26)
+    f.setOption(cfb.OPT_CHAIN_HISTOGRAM, 1)
+    d = dev(orc.splitmix64(331, int(0.9 * f.capacity())))
+    n = d.numel()
+    s = torch.cuda.Stream()
+    f.insertMany(d)  # the workspace exists
+    reads = {"occupied": lambda: f.occupiedSlots() == n,
+             "slots": lambda: f.countOccupiedSlots() == n,
+             "stats": lambda: (lambda st: st["primary"] + st["secondary"] + st["evicted_inserts"] == n)(f.stats()),
+             "chains": lambda: int(f.chainHistogram().sum()) == f.stats()["evicted_inserts"] > 0,
+             "reset": lambda: f.resetEvictionCount() is None and f.evictionCount() == 0}
+    for name, read in reads.items():
+        f.clear()
+        torch.cuda.synchronize()
+        f.insertManyAsync(d, stream=s)
+        assert read(), name
+        torch.cuda.synchronize()
+        assert f.occupiedSlots() == n and (name != "reset" or f.evictionCount() == 0)
+    f.close()
+
+
 def test_staged_batches_of_several_threads(cfb, orc):
     """Threads that insert and delete staged batches of one filter at the same time, the
     workspace growing between them; every count lies between what other threads can leave."""
