@@ -123,6 +123,30 @@ __device__ __forceinline__ void bin_copy(void* dst, const void* src) {
 }
 __device__ __forceinline__ void bin_copies_done() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
+// An entry (bucket b, tag) that finds no room in its bin goes to the eviction list:
+// one atomic for the lanes that come here together (with one each, the lists of
+// batches full of repeated keys were bound by it).  Not inlined: few batches have any.
+template <class C, bool PAY, typename EO>
+__device__ __noinline__ void bin_no_room(const BinArgs<EO>& a, uint64_t b, uint32_t tag, uint32_t pay) {
+    if (a.over_alt) {
+        b = alt_bucket<C>(b, tag, a.nb_mask);
+        tag = alt_tag<C>(tag);
+    }
+    const uint32_t lanes = __activemask(), lane = threadIdx.x & 31;
+    unsigned long long to = 0;
+    if (lane == static_cast<uint32_t>(__ffs(lanes)) - 1u)
+        to = atomicAdd(a.over_count, static_cast<unsigned long long>(__popc(lanes)));
+    to = __shfl_sync(lanes, to, __ffs(lanes) - 1) + __popc(lanes & ((1u << lane) - 1u));
+    if (to < a.over_room) {
+        a.over[to] = pack_entry<C>(b, tag);
+        if constexpr (PAY) a.over_pay[to] = pay;
+    } else if (a.ctr) {
+        atomicAdd(a.over_count, ~0ull);  // the list stays full: a failed insert
+        atomicAdd(&a.ctr[CTR_FAILED], 1ull);
+        if constexpr (PAY) a.out[pay] = 0;
+    }
+}
+
 // One binning pass.  A tile of kBinThreads * IPT entries is ranked within its
 // bins by shared-memory atomics, its runs' places are taken from the bins'
 // cursors, and the tile is staged in bin order and written out run by run.
@@ -142,7 +166,7 @@ __device__ __forceinline__ void bin_copies_done() { asm volatile("cp.async.wait_
 // Three CTAs of 40 registers with 7 entries per thread, or 256-thread CTAs, came
 // within 3 %; hashing before the staging instead of between it cost 10 %.
 template <class C, int SRC, typename EI, typename EO, bool PAY, int IPT>
-__global__ void __launch_bounds__(kBinThreads, 2) k_bin(BinArgs<EO> a) {
+__global__ void __launch_bounds__(kBinThreads, 2) k_bin(const __grid_constant__ BinArgs<EO> a) {
     constexpr int NT = kBinThreads;
     constexpr uint32_t TILE = NT * IPT;
     constexpr bool WIDE = sizeof(EO) == 8;
@@ -337,21 +361,9 @@ __global__ void __launch_bounds__(kBinThreads, 2) k_bin(BinArgs<EO> a) {
             const EO e = WIDE ? static_cast<EO>(y & wide_mask) : static_cast<EO>(y);
             const uint32_t o = word_at(base, d4) + q;
             if (check && o - (bin0 + d4 / 4) * a.dst_cap >= a.dst_cap) {  // no room left in its bin
-                uint64_t b = (static_cast<uint64_t>(bin0 + d4 / 4) << a.low) | (static_cast<uint64_t>(e) >> C::bits);
-                uint32_t tag = static_cast<uint32_t>(e) & C::tag_mask;
-                if (a.over_alt) {
-                    b = alt_bucket<C>(b, tag, a.nb_mask);
-                    tag = alt_tag<C>(tag);
-                }
-                const unsigned long long to = atomicAdd(a.over_count, 1ull);
-                if (to < a.over_room) {
-                    a.over[to] = pack_entry<C>(b, tag);
-                    if constexpr (PAY) a.over_pay[to] = stage_pay[q];
-                } else if (a.ctr) {
-                    atomicAdd(a.over_count, ~0ull);  // the list stays full: a failed insert
-                    atomicAdd(&a.ctr[CTR_FAILED], 1ull);
-                    if constexpr (PAY) a.out[stage_pay[q]] = 0;
-                }
+                const uint64_t b = (static_cast<uint64_t>(bin0 + d4 / 4) << a.low) | (static_cast<uint64_t>(e) >> C::bits);
+                const uint32_t tag = static_cast<uint32_t>(e) & C::tag_mask;
+                bin_no_room<C, PAY>(a, b, tag, PAY ? stage_pay[q] : 0u);
             } else {
                 a.dst[o] = e;
                 if constexpr (PAY) a.dst_pay[o] = stage_pay[q];
@@ -575,15 +587,15 @@ __global__ void __launch_bounds__(kBinInsertThreads, 3)
     if (tid == 0) bulk_wait_all();
 }
 
-// The entries that found no room in a bin, keyed by alternate bucket: a whole
-// insert each (either bucket, else eviction), since neither has been tried.
+// The entries that found no room in a bin, keyed by alternate bucket: neither
+// bucket has been tried, so both are; a stored key's entry is zeroed, the others
+// stay in the list for the eviction kernels, which take many more keys at a time
+// (evicting here, a thread per key: fills of 2^26 slots to 0.6 with half the batch
+// repeats of 10^4 keys, BFS, 351 ms; 257 like this, 272 segment-staged).
 template <class C>
-__global__ void __launch_bounds__(256) k_bin_over(DevTable t, const uint64_t* ent, const uint32_t* pay,
-                                                  const unsigned long long* n_dev, uint32_t policy_bfs, uint32_t max_ev,
-                                                  uint8_t* fail_out) {
+__global__ void __launch_bounds__(256) k_bin_over(DevTable t, uint64_t* ent, const unsigned long long* n_dev) {
     const uint64_t m = *n_dev;
-    uint32_t n_prim = 0, n_sec = 0, n_evk = 0, n_fail = 0;
-    EvictStats st;
+    uint32_t n_prim = 0, n_sec = 0;
     bool err = false;
     for (uint64_t i = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x; i < m;
          i += static_cast<uint64_t>(gridDim.x) * blockDim.x) {
@@ -595,35 +607,19 @@ __global__ void __launch_bounds__(256) k_bin_over(DevTable t, const uint64_t* en
         load_rlx<C::bucket_bytes>(bw, c);
         if (try_insert<C>(bw, c, fp1, err)) {
             ++n_prim;
+            ent[i] = 0;
             continue;
         }
         bw = bucket_words<C>(t, i2);
         load_rlx<C::bucket_bytes>(bw, c);
         if (try_insert<C>(bw, c, fp2, err)) {
             ++n_sec;
-            continue;
-        }
-        const bool even = (fp2 & 1u) == 0;  // the Offset policy's choice bit is the top bit
-        const uint32_t before = st.evictions;
-        ++n_evk;
-        const bool ok = policy_bfs
-            ? evict_bfs<C>(t, even ? fp1 : fp2, even ? i1 : i2, even ? i2 : i1, max_ev, st, err)
-            : evict_dfs<C>(t, even ? fp1 : fp2, even ? i1 : i2, even ? i2 : i1, max_ev, st, err);
-        if (ok) {
-            record_chain(t, st.evictions - before);
-        } else {
-            ++n_fail;
-            if (fail_out) fail_out[pay[i]] = 0;
+            ent[i] = 0;
         }
     }
-    flush_counters(t.ctr, {{CTR_OCCUPIED, static_cast<int32_t>(n_prim + n_sec + n_evk - n_fail - st.lost + st.dup)},
+    flush_counters(t.ctr, {{CTR_OCCUPIED, static_cast<int32_t>(n_prim + n_sec)},
                            {CTR_PRIMARY, static_cast<int32_t>(n_prim)},
-                           {CTR_SECONDARY, static_cast<int32_t>(n_sec)},
-                           {CTR_DUP, static_cast<int32_t>(st.dup)},
-                           {CTR_EVICTED_INSERTS, static_cast<int32_t>(n_evk)},
-                           {CTR_EVICTIONS, static_cast<int32_t>(st.evictions)},
-                           {CTR_FAILED, static_cast<int32_t>(n_fail)},
-                           {CTR_LOST, static_cast<int32_t>(st.lost)}});
+                           {CTR_SECONDARY, static_cast<int32_t>(n_sec)}});
     if (__any_sync(0xFFFFFFFFu, err) && (threadIdx.x & 31) == 0) atomicOr(&t.ctr[CTR_ERROR], ERR_CAS_LIMIT);
 }
 

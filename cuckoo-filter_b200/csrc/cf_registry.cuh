@@ -456,26 +456,28 @@ struct Launchers {
         return cudaGetLastError();
     }
 
-    // Eviction of a list of keys whose buckets were full; `rest` is a second
-    // buffer of the list's size, and the list starts at entry *first (0 when null).  BFS: a lockstep pass over the first candidates,
-    // then the step machine for what it could not place, then DFS.
+    // Eviction of a list of keys whose buckets were full (*count entries and *more
+    // more, zero where a key has been stored meanwhile); `rest` is a second buffer of
+    // the list's size.  BFS: a lockstep pass over the first candidates, then the step
+    // machine for what it could not place, then DFS.
     static void evict_left(const DevTable& t, uint64_t* list, uint32_t* list_pay, const unsigned long long* count,
                            uint64_t* rest, uint32_t* rest_pay, unsigned long long* rest_count,
                            unsigned long long* dfs_count, uint32_t* bitmap, uint8_t* fail_out, uint32_t* full, int sms,
                            cudaStream_t s, uint32_t policy_bfs, uint32_t max_ev,
-                           const unsigned long long* first = nullptr, uint64_t batch = UINT64_MAX) {
+                           const unsigned long long* more = nullptr, uint64_t batch = UINT64_MAX) {
         static const int list_bps = blocks_per_sm(k_evict_list<C>, 256, 0);
         if (!policy_bfs) {
             { k_evict_list<C><<<sms * list_bps * kEvictGridWaves, 256, 0, s>>>(t, list, list_pay, count, 0u, max_ev, bitmap,
-                                                                              0u, fail_out, first); CF_COUNT_LAUNCH(); }
+                                                                              0u, fail_out, more); CF_COUNT_LAUNCH(); }
             return;
         }
         if constexpr (C::bs <= 16) {
             if (!bitmap && batch <= kCoopEvictBatch) {
-                { k_evict_bfs_coop<C><<<sms * 4, 256, 0, s>>>(t, list, list_pay, count, first, rest, rest_pay, dfs_count, full);
+                { k_evict_bfs_coop<C><<<sms * 4, 256, 0, s>>>(t, list, list_pay, count, more, rest, rest_pay, dfs_count, full);
                   CF_COUNT_LAUNCH(); }
-                { k_evict_list<C><<<sms * 2, 256, 0, s>>>(t, rest, rest_pay, dfs_count, 0u, max_ev, bitmap, 1u, fail_out,
-                                                          nullptr); CF_COUNT_LAUNCH(); }
+                // one wave: the list is usually short, but that of a batch full of repeated keys is not
+                { k_evict_list<C><<<sms * list_bps, 256, 0, s>>>(t, rest, rest_pay, dfs_count, 0u, max_ev, bitmap, 1u, fail_out,
+                                                                nullptr); CF_COUNT_LAUNCH(); }
                 return;
             }
         }
@@ -485,7 +487,7 @@ struct Launchers {
         const int bucket_bits = t.nb_mask ? 64 - __builtin_clzll(t.nb_mask) : 0;
         const uint32_t flag_ok = bucket_bits + C::bits <= 63 ? 1u : 0u;
         { k_evict_bfs_fast<C, kBfsFastProbes><<<sms * fast_bps * kEvictGridWaves, 256, 0, s>>>(
-              t, list, list_pay, count, bitmap, rest, rest_pay, rest_count, full, flag_ok, first); CF_COUNT_LAUNCH(); }
+              t, list, list_pay, count, bitmap, rest, rest_pay, rest_count, full, flag_ok, more); CF_COUNT_LAUNCH(); }
         { k_evict_bfs_steps<C><<<sms * bfs_bps * kEvictGridWaves, 256, 0, s>>>(t, rest, rest_pay, rest_count, bitmap, list,
                                                                               list_pay, dfs_count, 0u); CF_COUNT_LAUNCH(); }
         { k_evict_list<C><<<sms * list_bps * kEvictGridWaves, 256, 0, s>>>(t, list, list_pay, dfs_count, 0u, max_ev, bitmap,
@@ -616,8 +618,7 @@ struct Launchers {
             e = cudaGetLastError();
         }
         if (e != cudaSuccess) return e;
-        { k_bin_over<C><<<w.sms * 2, 256, 0, s>>>(t, w.list, w.list_pay, &w.cnt[0], policy_bfs, max_ev,
-                                                 PAY ? out : nullptr); CF_COUNT_LAUNCH(); }
+        { k_bin_over<C><<<w.sms * 4, 256, 0, s>>>(t, w.list, &w.cnt[0]); CF_COUNT_LAUNCH(); }
         evict_left(t, w.list, w.list_pay, &w.cnt[3], w.list + m, PAY ? w.list_pay + m : nullptr, &w.cnt[1], &w.cnt[2],
                    nullptr, PAY ? out : nullptr, w.full, w.sms, s, policy_bfs, max_ev, &w.cnt[0], m);
         return cudaGetLastError();

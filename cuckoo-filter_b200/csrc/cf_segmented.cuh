@@ -898,33 +898,30 @@ __device__ __forceinline__ uint32_t empty_count(const uint64_t (&c)[C::nchunks])
 // step machine when flag_ok, else through it); a key that used its P probes,
 // or whose compare-and-swap found a bucket changed, goes to `rest`, where the
 // step-machine BFS starts it over.  One key alone takes the reference's steps.
+// The list has *n_dev entries and *more_dev more (none when null), zero where a
+// key has been stored meanwhile (k_bin_over), here and in the two kernels below.
 template <class C, int P>
 __global__ void __launch_bounds__(256, C::nchunks <= 4 ? 3 : 2) k_evict_bfs_fast(DevTable t, const uint64_t* ent, const uint32_t* pay,
                                                         const unsigned long long* n_dev, uint32_t* bitmap,
                                                         uint64_t* rest, uint32_t* rest_pay,
                                                         unsigned long long* rest_count, uint32_t* full,
-                                                        uint32_t flag_ok, const unsigned long long* first_dev) {
+                                                        uint32_t flag_ok, const unsigned long long* more_dev) {
     constexpr uint64_t lane_mask = C::bits == 32 ? 0xFFFFFFFFULL : ((1ULL << C::bits) - 1ULL);
     constexpr int NC = (C::bs / 2) < 8 ? (C::bs / 2) : 8;
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t lt_mask = (1u << lane) - 1u;
-    if (first_dev) {
-        ent += *first_dev;
-        if (pay) pay += *first_dev;
-    }
-    const uint64_t m = *n_dev;
+    const uint64_t m = *n_dev + (more_dev ? *more_dev : 0ull);
     uint32_t n_evk = 0, n_ok = 0, n_ev = 0, n_dup = 0;
     bool err = false;
     const uint64_t stride = static_cast<uint64_t>(gridDim.x) * blockDim.x;
     // warp-uniform trip count: every lane reaches the ballot below
     for (uint64_t base = static_cast<uint64_t>(blockIdx.x) * blockDim.x; base < m; base += stride) {
         const uint64_t i = base + threadIdx.x;
-        const bool v = i < m;
         bool done = false, stop = false;
-        uint64_t e = 0;
+        uint64_t e = i < m ? __ldcs(reinterpret_cast<const unsigned long long*>(ent) + i) : 0ull;
+        const bool v = e != 0;
         if (v) {
             ++n_evk;
-            e = __ldcs(reinterpret_cast<const unsigned long long*>(ent) + i);
             const uint32_t fp0 = static_cast<uint32_t>(e) & C::tag_mask;
             const uint64_t i2 = e >> C::bits;
             const uint64_t i1 = alt_bucket<C>(i2, fp0, t.nb_mask);
@@ -1038,7 +1035,7 @@ constexpr int kCoopTries = 16;
 template <class C>
 __global__ void __launch_bounds__(256) k_evict_bfs_coop(DevTable t, const uint64_t* ent, const uint32_t* pay,
                                                         const unsigned long long* n_dev,
-                                                        const unsigned long long* first_dev, uint64_t* dfs,
+                                                        const unsigned long long* more_dev, uint64_t* dfs,
                                                         uint32_t* dfs_pay, unsigned long long* dfs_count,
                                                         const uint32_t* full) {
     constexpr uint64_t lane_mask = C::bits == 32 ? 0xFFFFFFFFULL : ((1ULL << C::bits) - 1ULL);
@@ -1046,18 +1043,18 @@ __global__ void __launch_bounds__(256) k_evict_bfs_coop(DevTable t, const uint64
     static_assert(NC >= 1 && 32 % NC == 0, "a group of NC lanes per key");
     const uint32_t lane = threadIdx.x & 31, q = lane % NC;
     const uint32_t gmask = (NC == 32 ? 0xFFFFFFFFu : (1u << NC) - 1u) << (lane - q);
-    const uint64_t m = *n_dev, first = first_dev ? *first_dev : 0ull;
+    const uint64_t m = *n_dev + (more_dev ? *more_dev : 0ull);
     uint32_t n_evk = 0, n_ok = 0, n_ev = 0, n_dup = 0;
     bool err = false;
     const uint64_t step = static_cast<uint64_t>(gridDim.x) * (blockDim.x / NC);
     // the trip count is uniform over the CTA: every lane reaches every vote
     for (uint64_t base = static_cast<uint64_t>(blockIdx.x) * (blockDim.x / NC); base < m; base += step) {
         const uint64_t i = base + threadIdx.x / NC;
-        const bool v = i < m;
+        const uint64_t e = i < m ? ent[i] : 0ull;
+        const bool v = e != 0;
         bool pend = v, done = false;
         uint64_t start = 0;
         uint32_t fp = 0;
-        const uint64_t e = v ? ent[first + i] : 0ull;
         if (v) {
             n_evk += q == 0;
             const uint32_t fp0 = static_cast<uint32_t>(e) & C::tag_mask;
@@ -1117,7 +1114,7 @@ __global__ void __launch_bounds__(256) k_evict_bfs_coop(DevTable t, const uint64
         if (v && !done && q == 0) {
             const unsigned long long o = atomicAdd(dfs_count, 1ull);
             dfs[o] = e;
-            if (dfs_pay) dfs_pay[o] = pay[first + i];
+            if (dfs_pay) dfs_pay[o] = pay[i];
         }
     }
     flush_counters(t.ctr, {{CTR_OCCUPIED, static_cast<int32_t>(n_ok + n_dup)},
@@ -1131,23 +1128,19 @@ __global__ void __launch_bounds__(256) k_evict_bfs_coop(DevTable t, const uint64
 // (or, with `continued`, whose BFS candidates all failed); entries carry
 // (alternate bucket, tag).  One key per thread, all lanes busy.  Results: a
 // stored key's bit is set in `bitmap`, or a failed key's byte cleared in `fail_out`.
-// The list starts at entry *first_dev (0 when null).
 template <class C>
 __global__ void __launch_bounds__(256) k_evict_list(DevTable t, const uint64_t* ent, const uint32_t* pay,
                                                     const unsigned long long* n_dev, uint32_t policy_bfs,
                                                     uint32_t max_ev, uint32_t* bitmap, uint32_t continued,
-                                                    uint8_t* fail_out, const unsigned long long* first_dev) {
-    if (first_dev) {
-        ent += *first_dev;
-        if (pay) pay += *first_dev;
-    }
-    const uint64_t m = *n_dev;
+                                                    uint8_t* fail_out, const unsigned long long* more_dev) {
+    const uint64_t m = *n_dev + (more_dev ? *more_dev : 0ull);
     uint32_t n_evk = 0, n_fail = 0;
     EvictStats st;
     bool err = false;
     for (uint64_t i = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x; i < m;
          i += static_cast<uint64_t>(gridDim.x) * blockDim.x) {
         const uint64_t e = ent[i];
+        if (!e) continue;
         const uint32_t fp = static_cast<uint32_t>(e) & C::tag_mask;
         const uint64_t i2 = e >> C::bits;
         const uint64_t i1 = alt_bucket<C>(i2, fp, t.nb_mask);

@@ -162,6 +162,37 @@ def test_binned_insert_of_repeated_keys(cfb, orc, kb, bits, bs, slots, hot, copi
     f.close()
 
 
+@pytest.mark.parametrize("results", [False, True])
+@pytest.mark.parametrize("bits,slots,n,copies,dfs", [
+    (16, 1 << 16, 9000, 5000, True),             # walks over a short list
+    (16, 1 << 24, 3 << 20, 1 << 20, True),
+    (8, 1 << 20, 1 << 19, 1 << 18, False),       # eviction lanes
+    (8, 1 << 27, (1 << 25) + 4096, 5000, False), # the lockstep pass
+])
+def test_binned_insert_evicts_beside_stored_entries(cfb, orc, bits, slots, n, copies, dfs, results):
+    """The eviction kernels on a list where entries without room in a bin have been
+    stored (and zeroed) between ones that have not."""
+    cfg = cfb.CuckooConfig(T="uint64", bitsPerTag=bits, bucketSize=16, maxEvictions=4,
+                           evictionPolicy=cfb.EvictionPolicy.DFS if dfs else cfb.EvictionPolicy.BFS)
+    f = cfb.CuckooFilter(cfg, slots)
+    rest = dev(orc.splitmix64(41, n))
+    hot = dev(orc.splitmix64(42, 1))
+    near = f.getNumBuckets() // 256  # keys of the repeated key's segment at least get no room in its bin
+    keys = torch.cat([hot.expand(copies), rest])
+    keys = keys[torch.randperm(keys.numel(), device="cuda", generator=torch.Generator("cuda").manual_seed(near))].contiguous()
+    ok = torch.zeros(keys.numel(), dtype=torch.bool, device="cuda") if results else None
+    occ = f.insertMany(keys, d_output=ok)
+    st = f.stats()
+    assert occ == f.countOccupiedSlots() == keys.numel() - st["failed"] - st["lost"] + st["duplicates"]
+    assert st["primary"] + st["secondary"] + st["evicted_inserts"] == keys.numel()
+    assert copies - 32 - st["lost"] <= st["failed"] <= copies
+    assert ok is None or int(ok.sum()) == keys.numel() - st["failed"]
+    assert bool(f.containsMany(hot).all())
+    if st["lost"] == 0:
+        assert bool(f.containsMany(rest).all())
+    f.close()
+
+
 @pytest.mark.parametrize("bits,bs", [(8, 16), (16, 16), (32, 8)])
 @pytest.mark.parametrize("kpt", [1, 2, 4, 8])
 def test_set_items_that_end_inside_a_thread(cfb, orc, bits, bs, kpt):
