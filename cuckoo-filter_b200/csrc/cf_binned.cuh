@@ -15,7 +15,8 @@
 //            primary bucket again; what is left goes to the eviction kernels.
 //
 // Every count stays on the device: the host enqueues all launches of a batch
-// and waits for none of them.  Used for batches whose slot order within a bucket
+// and waits for none of them, unless the list is shorter than the batch (two waits,
+// see list_room).  Used for batches whose slot order within a bucket
 // is unspecified, in buckets of at most 16 slots; cf_segmented.cuh takes the rest.
 #pragma once
 
@@ -57,14 +58,16 @@ struct BinWork {
     // found no room in a bin (at most list_room of them), then the last round's.
     // list, ent[0] and ent[1] lie one after the other: with list_room below the
     // batch size (two passes only) the list runs on into ent[0], which is free
-    // in the last round, and its second buffer starts m entries in.
+    // in the last round, and its second buffer starts m entries in.  Such a list
+    // never fills up: past it in the first round the batch is given up, and
+    // entries the first round leaves are binned again only where all would fit.
     uint64_t* list;
     uint32_t* list_pay;
     uint64_t list_room;
     unsigned long long* h_cnt;   // pinned
     uint32_t* cursor;            // per round: d1 (two passes) and nseg entry counts
     uint32_t* left;              // per segment: entries left by the round
-    unsigned long long* cnt;     // list lengths: no room in a bin, after the fast BFS, after BFS, the last round's
+    unsigned long long* cnt;     // list lengths: no room in a bin, after the fast BFS, after BFS, the last round's; left by the first round
     uint32_t* full;              // known-full bucket bitmap, or null
     uint64_t zero_bytes;         // cursor, cnt and full, one after the other: zero at the start of a batch
     int sms;
@@ -91,9 +94,7 @@ struct BinArgs {
     uint64_t* over;             // entries without room, keyed by alternate bucket
     uint32_t* over_pay;
     unsigned long long* over_count;
-    uint64_t over_room;         // entries the list holds
-    uint8_t* out;               // per-key results, or null
-    unsigned long long* ctr;    // counters: an entry past over_room is a failed insert (null: it is only counted)
+    uint64_t over_room;         // entries the list holds (past it, in the first round only, they are counted)
     int over_alt;               // the entries binned here are keyed by primary bucket
 };
 
@@ -140,10 +141,6 @@ __device__ __noinline__ void bin_no_room(const BinArgs<EO>& a, uint64_t b, uint3
     if (to < a.over_room) {
         a.over[to] = pack_entry<C>(b, tag);
         if constexpr (PAY) a.over_pay[to] = pay;
-    } else if (a.ctr) {
-        atomicAdd(a.over_count, ~0ull);  // the list stays full: a failed insert
-        atomicAdd(&a.ctr[CTR_FAILED], 1ull);
-        if constexpr (PAY) a.out[pay] = 0;
     }
 }
 
@@ -585,6 +582,36 @@ __global__ void __launch_bounds__(kBinInsertThreads, 3)
     flush_counters(t.ctr, {{round == 2 ? CTR_SECONDARY : CTR_PRIMARY, static_cast<int32_t>(n_ok)},
                            {CTR_OCCUPIED, static_cast<int32_t>(n_ok)}});
     if (tid == 0) bulk_wait_all();
+}
+
+// Adds the entries that a round left in its segments' bins to *total.
+static __global__ void __launch_bounds__(256) k_bin_left(const uint32_t* left, uint32_t nseg, unsigned long long* total) {
+    uint32_t n = 0;
+    for (uint32_t s = blockIdx.x * blockDim.x + threadIdx.x; s < nseg; s += gridDim.x * blockDim.x) n += left[s];
+    flush_counters(total, {{0, static_cast<int32_t>(n)}});
+}
+
+// Moves them to the list instead, keyed by alternate bucket: a warp per segment.
+// For a list of half the batch that the next rounds might fill.
+template <class C, typename E, bool PAY>
+__global__ void __launch_bounds__(256) k_bin_to_list(const E* ent, const uint32_t* pay, const uint32_t* left, uint32_t room,
+                                                     uint32_t nseg, int sbl, uint64_t nb_mask, uint64_t* list,
+                                                     uint32_t* list_pay, unsigned long long* list_count) {
+    const uint32_t lane = threadIdx.x & 31, nwarps = gridDim.x * (blockDim.x / 32);
+    for (uint32_t s = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32; s < nseg; s += nwarps) {
+        const uint32_t n = left[s];
+        if (n == 0) continue;
+        unsigned long long base = 0;
+        if (lane == 0) base = atomicAdd(list_count, static_cast<unsigned long long>(n));
+        base = __shfl_sync(0xFFFFFFFFu, base, 0);
+        for (uint32_t k = lane; k < n; k += 32) {
+            const E e = ent[static_cast<uint64_t>(s) * room + k];
+            const uint32_t tag = static_cast<uint32_t>(e) & C::tag_mask;
+            const uint64_t b = (static_cast<uint64_t>(s) << sbl) | (static_cast<uint64_t>(e) >> C::bits);
+            list[base + k] = pack_entry<C>(alt_bucket<C>(b, tag, nb_mask), alt_tag<C>(tag));
+            if constexpr (PAY) list_pay[base + k] = pay[static_cast<uint64_t>(s) * room + k];
+        }
+    }
 }
 
 // The entries that found no room in a bin, keyed by alternate bucket: neither

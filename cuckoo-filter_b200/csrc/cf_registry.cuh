@@ -540,6 +540,12 @@ struct Launchers {
         constexpr int kMaxSmem = kSegBytes + kSegBytes / C::bucket_bytes * 4;
         if (e == cudaSuccess) e = ensure_smem_attr<k_bin_insert<C, E2, PAY, true>>(kMaxSmem);
         if (e == cudaSuccess) e = ensure_smem_attr<k_bin_insert<C, E2, PAY, false>>(kMaxSmem);
+        const bool short_list = w.list_room < m;
+        auto read_back = [&](const unsigned long long* c) {  // -> *w.h_cnt
+            cudaError_t st = cudaMemcpyAsync(w.h_cnt, c, sizeof(unsigned long long), cudaMemcpyDeviceToHost, s);
+            return st == cudaSuccess ? cudaStreamSynchronize(s) : st;
+        };
+        uint64_t over = 0;
         int at = 0;  // the buffer of the segments' bins
         for (int r = 1; r <= rounds && e == cudaSuccess; ++r) {
             uint32_t* cur = w.cursor + static_cast<size_t>(per_round) * (r - 1);
@@ -555,8 +561,6 @@ struct Launchers {
                 a.over_pay = w.list_pay;
                 a.over_count = &w.cnt[0];
                 a.over_room = w.list_room;
-                a.out = out;
-                a.ctr = r == 1 ? nullptr : t.ctr;
                 a.over_alt = r != 2;
                 if (first) {
                     a.src = w.ent[at];
@@ -595,13 +599,12 @@ struct Launchers {
                 at = 1 - to;
             }
             if (e != cudaSuccess) break;
-            if (r == 1 && w.list_room < m) {
-                // the list is shorter than the batch: a batch too skewed for it
-                // is left to the segment-staged path (nothing is stored yet)
-                e = cudaMemcpyAsync(w.h_cnt, &w.cnt[0], sizeof(unsigned long long), cudaMemcpyDeviceToHost, s);
-                if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-                if (e != cudaSuccess) break;
-                *skewed = w.h_cnt[0] > w.list_room;
+            if (r == 1 && short_list) {
+                // a batch too skewed for the list is left to the segment-staged
+                // path (nothing is stored yet)
+                if ((e = read_back(&w.cnt[0])) != cudaSuccess) break;
+                over = *w.h_cnt;
+                *skewed = over > w.list_room;
                 if (*skewed) return cudaSuccess;
             }
             E2* ent = static_cast<E2*>(w.ent[at]);
@@ -616,6 +619,20 @@ struct Launchers {
                       t, ent, w.pay[at], seg_count, g.room2, g.nseg, g.sbl, r, w.left, cap, last, w.list, w.list_pay,
                       &w.cnt[3], &w.cnt[0], w.full); CF_COUNT_LAUNCH(); }
             e = cudaGetLastError();
+            if (e == cudaSuccess && r == 1 && short_list) {
+                // what this round left could fill the list if it does not hash evenly
+                // either: where it might not fit, it goes there now (then the list holds
+                // at most the whole batch, and ent[0] is free) and is inserted at random
+                { k_bin_left<<<w.sms, 256, 0, s>>>(w.left, g.nseg, &w.cnt[4]); CF_COUNT_LAUNCH(); }
+                if ((e = cudaGetLastError()) != cudaSuccess || (e = read_back(&w.cnt[4])) != cudaSuccess) break;
+                if (over + *w.h_cnt > w.list_room) {
+                    { k_bin_to_list<C, E2, PAY><<<w.sms * 4, 256, 0, s>>>(ent, w.pay[at], w.left, g.room2, g.nseg, g.sbl,
+                                                                          t.nb_mask, w.list, w.list_pay, &w.cnt[0]);
+                      CF_COUNT_LAUNCH(); }
+                    e = cudaGetLastError();
+                    break;
+                }
+            }
         }
         if (e != cudaSuccess) return e;
         { k_bin_over<C><<<w.sms * 4, 256, 0, s>>>(t, w.list, &w.cnt[0]); CF_COUNT_LAUNCH(); }

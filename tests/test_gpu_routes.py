@@ -193,6 +193,37 @@ def test_binned_insert_evicts_beside_stored_entries(cfb, orc, bits, slots, n, co
     f.close()
 
 
+@pytest.mark.parametrize("results,limit", [(False, 49 << 20), (True, 66 << 20)])
+@pytest.mark.parametrize("dfs", [False, True])
+def test_binned_insert_past_a_half_length_list(cfb, orc, results, limit, dfs):
+    """A list of half the batch that is long enough for the first round and not for
+    the second: every key's primary bucket is full, and every alternate bucket
+    lies in a quarter of the table that is empty and has room for all of them."""
+    cfg = cfb.CuckooConfig(T="uint64", bitsPerTag=32, bucketSize=8, maxEvictions=100,
+                           evictionPolicy=cfb.EvictionPolicy.DFS if dfs else cfb.EvictionPolicy.BFS)
+    f = cfb.CuckooFilter(cfg, 1 << 24)
+    nb = f.getNumBuckets()
+    image = np.zeros((nb, 8), np.uint32)
+    image[nb // 4:] = np.arange(1, 6 * nb + 1, dtype=np.uint32).reshape(-1, 8) | np.uint32(1)
+    f.load_table(torch.from_numpy(image.view(np.uint8).reshape(-1)).cuda())
+    full = f.occupiedSlots()
+    assert full == 6 * nb
+    pool = orc.splitmix64(51, 12 << 20)
+    i1, i2, _ = cfb.CuckooFilter.getCandidateBuckets(cfg, pool, nb)
+    keys = pool[(i1 >= nb // 4) & (i2 < nb // 4)]
+    assert len(keys) >= nb
+    d = dev(keys[:nb])
+    f.setOption(cfb.OPT_WORKSPACE_LIMIT, limit)
+    ok = torch.zeros(nb, dtype=torch.bool, device="cuda") if results else None
+    occ = f.insertMany(d, d_output=ok)
+    st = f.stats()
+    assert occ == full + nb == f.countOccupiedSlots() and st["failed"] == st["lost"] == st["duplicates"] == 0, st
+    assert st["primary"] + st["secondary"] + st["evicted_inserts"] == nb
+    assert ok is None or bool(ok.all())
+    assert bool(f.containsMany(d).all())
+    f.close()
+
+
 @pytest.mark.parametrize("bits,bs", [(8, 16), (16, 16), (32, 8)])
 @pytest.mark.parametrize("kpt", [1, 2, 4, 8])
 def test_set_items_that_end_inside_a_thread(cfb, orc, bits, bs, kpt):
