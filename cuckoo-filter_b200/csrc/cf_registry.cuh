@@ -635,7 +635,7 @@ struct Launchers {
             }
         }
         if (e != cudaSuccess) return e;
-        { k_bin_over<C><<<w.sms * 4, 256, 0, s>>>(t, w.list, &w.cnt[0]); CF_COUNT_LAUNCH(); }
+        { k_bin_over<C><<<w.sms * 2, 256, 0, s>>>(t, w.list, &w.cnt[0]); CF_COUNT_LAUNCH(); }
         evict_left(t, w.list, w.list_pay, &w.cnt[3], w.list + m, PAY ? w.list_pay + m : nullptr, &w.cnt[1], &w.cnt[2],
                    nullptr, PAY ? out : nullptr, w.full, w.sms, s, policy_bfs, max_ev, &w.cnt[0], m);
         return cudaGetLastError();
