@@ -567,22 +567,30 @@ struct CounterAdd {
     int idx;
     int32_t v;
 };
+// A thread's part has 32 bits, the sums 64: the evictions of a CTA's failing keys
+// (up to 512 each) do not fit fewer.
 template <int N>
 __device__ __forceinline__ void flush_counters(unsigned long long* ctr, const CounterAdd (&a)[N]) {
-    __shared__ int32_t s_part[N][32];
+    static_assert(N <= 32, "lane i adds counter i");
+    __shared__ long long s_part[32][N];
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = (blockDim.x + 31) >> 5;
 #pragma unroll
     for (int i = 0; i < N; ++i) {
-        const int32_t s = __reduce_add_sync(0xFFFFFFFFu, a[i].v);
-        if (lane == 0) s_part[i][warp] = s;
+        const int32_t hi = __reduce_add_sync(0xFFFFFFFFu, a[i].v >> 16);
+        const uint32_t lo = __reduce_add_sync(0xFFFFFFFFu, static_cast<uint32_t>(a[i].v) & 0xFFFFu);
+        if (lane == 0) s_part[warp][i] = static_cast<long long>(hi) * 65536 + lo;
     }
     __syncthreads();
     if (warp != 0) return;
+    if (lane < N) {
+        int idx = 0;
+        long long s = 0;
 #pragma unroll
-    for (int i = 0; i < N; ++i) {
-        const int32_t s = __reduce_add_sync(0xFFFFFFFFu, lane < nwarp ? s_part[i][lane] : 0);
-        if (lane == 0 && s) atomicAdd(&ctr[a[i].idx], static_cast<unsigned long long>(static_cast<long long>(s)));
+        for (int i = 0; i < N; ++i) idx = static_cast<int>(lane) == i ? a[i].idx : idx;
+        for (uint32_t w = 0; w < nwarp; ++w) s += s_part[w][lane];
+        if (s) atomicAdd(&ctr[idx], static_cast<unsigned long long>(s));
     }
+    __syncwarp();
 }
 
 // After flush_counters: the last CTA of the grid to come here copies the counters
@@ -593,7 +601,7 @@ __device__ __forceinline__ void publish_counters(const DevTable& t) {
     if (!t.pub) return;
     __shared__ bool s_last;
     if (threadIdx.x == 0) {
-        __threadfence();  // this CTA's counter updates come before its ticket (thread 0's warp made them)
+        __threadfence();  // this CTA's counter updates come before its ticket (its warp made them)
         s_last = atomicAdd(t.ticket, 1u) == gridDim.x - 1;
     }
     __syncthreads();

@@ -542,6 +542,49 @@ def test_staged_batches_of_several_threads(cfb, orc):
     f.close()
 
 
+FLUSH = r"""
+#include <cstdio>
+#include "cf_kernels.cuh"
+__global__ void add(unsigned long long* ctr, int32_t big) {
+    const int32_t t = static_cast<int32_t>(threadIdx.x);
+    cfb::flush_counters(ctr, {{2, big - t}, {0, -big}, {1, (t & 1) ? 5 : -7}, {3, 0}});
+}
+int main() {
+    unsigned long long* c;
+    if (cudaMallocManaged(&c, 4 * sizeof *c) != cudaSuccess) return 2;
+    for (int threads : {32, 96, 256, 512, 1024})
+        for (int32_t big : {3, 1 << 30, 0x7fffffff}) {
+            for (int i = 0; i < 4; ++i) c[i] = 1000;
+            add<<<3, threads>>>(c, big);
+            if (cudaDeviceSynchronize() != cudaSuccess) return 3;
+            const long long n = 3ll * threads, tri = 3ll * threads * (threads - 1) / 2;
+            const long long want[4] = {1000 - n * big, 1000 - n, 1000 + n * big - tri, 1000};
+            for (int i = 0; i < 4; ++i)
+                if (static_cast<long long>(c[i]) != want[i])
+                    return printf("%d threads, counter %d: %lld, not %lld\n", threads, i, (long long)c[i], want[i]), 1;
+        }
+    return 0;
+}
+"""
+
+
+def test_counter_sums_past_32_bits(cfb, tmp_path):
+    """A CTA's sums of its threads' counts are exact however large and of whatever sign."""
+    import subprocess
+
+    pkg = os.path.dirname(cfb.__file__)
+    sys.path.insert(0, pkg)
+    import build
+
+    src, exe = tmp_path / "flush.cu", tmp_path / "flush"
+    src.write_text(FLUSH)
+    r = subprocess.run([build.nvcc(), *build.NVCC_FLAGS, "-I" + os.path.join(pkg, "csrc"), str(src), "-o", str(exe)],
+                       capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr
+    r = subprocess.run([str(exe)], capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0, r.stdout + r.stderr
+
+
 CAPTURE = """
 import __graft_entry__, oracle, torch
 cfb = __graft_entry__.package()
