@@ -890,9 +890,10 @@ int insert_any(cf_filter* f, const void* keys, uint64_t n, uint8_t* out, void* s
                 // against binned: 2^20 slots 420 -> 198 us, 2^28 6.58 -> 4.75 ms with a
                 // sample looked up, 2^31 45.8 -> 36.5 ms).  Buckets of more than 16
                 // slots, batches that do not fit the workspace limit in one piece and
-                // skewed ones with a short list stay segment-staged.
+                // skewed ones with a short list stay segment-staged, and so do those
+                // of a caller who asks for that path or sets an option of it.
                 bool taken = false;
-                if (n >= f->num_buckets)
+                if (n >= f->num_buckets && f->staging != CF_STAGING_SEGMENT && !f->round2_min)
                     if (int st = run_binned(f, keys, n, out, stream, &taken)) return st;
                 return taken ? CF_OK : run_segmented(f, SEG_INSERT, keys, n, out, stream);
             });

@@ -213,7 +213,9 @@ typedef enum cf_option {
     CF_OPT_WORKSPACE_LIMIT = 1,
     /* Batch size from which insertMany, containsMany and deleteMany stream
      * table segments through shared memory instead of probing at random
-     * (insertManySorted always does).  0 = automatic: one key per bucket for
+     * (insertManySorted always does): inserts of at least one key per bucket into
+     * buckets of at most 16 slots binned by segment in fixed places, if the
+     * workspace allows, everything else sorted by segment.  0 = automatic: one key per bucket for
      * inserts and at least 2^17 keys (2^20 when they cannot fill the table beyond
      * three quarters), eight per bucket for deletes, never for lookups (random
      * probes were faster at every size); UINT64_MAX = never. */
@@ -223,7 +225,8 @@ typedef enum cf_option {
     /* Inside a segment-staged batch: number of keys that missed their primary
      * bucket from which the alternate-bucket round is segment-staged too
      * (otherwise those keys are probed at random).  0 = automatic (table bytes
-     * / 64 for inserts, eight keys per bucket for lookups and deletes). */
+     * / 64 for inserts, eight keys per bucket for lookups and deletes); any other
+     * value keeps inserts from being binned. */
     CF_OPT_ROUND2_SEGMENTED_MIN_KEYS = 4,
     /* Batch size from which every operation is region-staged: the batch is
      * partitioned by ~16 MiB table region in one pass and applied region by
@@ -249,7 +252,7 @@ typedef enum cf_option {
      * (cf_get_chain_histogram); 0 = off (default; one atomic per evicting
      * insert when on). */
     CF_OPT_CHAIN_HISTOGRAM = 11,
-    /* Segment-staged inserts of at least one key per bucket: tags the first
+    /* Staged inserts of at least one key per bucket: tags the first
      * round (primary buckets) may leave in a bucket.  0 = automatic: 13 of
      * 16 slots (bucket_size minus 3/16 of it), the keys that miss their
      * primary and then their alternate bucket get a third round at the
@@ -281,8 +284,8 @@ int cf_get_chain_histogram(cf_filter* f, uint64_t* bins);
 /* Execution paths (CF_OPT_STAGING).  All give the same per-key results. */
 typedef enum cf_staging {
     CF_STAGING_AUTO = 0,
-    CF_STAGING_RANDOM = 1,  /* probe buckets at random, any batch size (insertManySorted: segment-staged) */
-    CF_STAGING_SEGMENT = 2, /* sort by 64 KiB segment, stage segments in shared memory */
+    CF_STAGING_RANDOM = 1,  /* probe buckets at random, any batch size (insertManySorted: as automatic) */
+    CF_STAGING_SEGMENT = 2, /* sort by 64 KiB segment, stage segments in shared memory (never binned) */
     CF_STAGING_REGION = 3   /* partition by ~16 MiB region, apply in region order through L2 */
 } cf_staging;
 

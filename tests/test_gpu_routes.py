@@ -193,6 +193,62 @@ def test_binned_insert_evicts_beside_stored_entries(cfb, orc, bits, slots, n, co
     f.close()
 
 
+def launches_of(cfb, f, call):
+    before = cfb.launch_count()
+    call()
+    return cfb.launch_count() - before
+
+
+def test_options_of_the_segment_path_are_obeyed(cfb, orc):
+    """CF_STAGING_SEGMENT and CF_OPT_ROUND2_SEGMENTED_MIN_KEYS select and steer the
+    segment-staged insert at one key per bucket and more, where automatic inserts are binned."""
+    cfg = cfb.CuckooConfig(T="uint64", bitsPerTag=16, bucketSize=16, evictionPolicy=cfb.EvictionPolicy.BFS)
+    f = cfb.CuckooFilter(cfg, 1 << 21)
+    d = dev(orc.splitmix64(341, int(0.8 * f.capacity())))
+    n = {}
+    for name, opts in {"auto": {}, "segment": {cfb.OPT_STAGING: cfb.STAGING_SEGMENT},
+                       "round2 staged": {cfb.OPT_ROUND2_SEGMENTED_MIN_KEYS: 1},
+                       "round2 random": {cfb.OPT_ROUND2_SEGMENTED_MIN_KEYS: cfb.NEVER}}.items():
+        f.clear()
+        for o, v in opts.items():
+            f.setOption(o, v)
+        n[name] = launches_of(cfb, f, lambda: f.insertMany(d))
+        assert f.countOccupiedSlots() == d.numel() and bool(f.containsMany(d).all())
+        f.setOption(cfb.OPT_STAGING, cfb.STAGING_AUTO)
+        f.setOption(cfb.OPT_ROUND2_SEGMENTED_MIN_KEYS, 0)
+    # one random pass in the place of two more sorted rounds and three eviction kernels
+    assert n["round2 random"] < n["round2 staged"] == n["segment"] != n["auto"], n
+    f.close()
+
+
+@pytest.mark.parametrize("dfs", [False, True])
+@pytest.mark.parametrize("results", [False, True])
+@pytest.mark.parametrize("kb,bits,bs,loads,limit", [
+    (8, 8, 16, (0.5, 0.4), 0), (8, 16, 16, (0.9,), 0), (4, 16, 16, (0.5, 0.4), 0), (8, 16, 4, (0.5, 0.35), 0),
+    (8, 8, 8, (0.9,), 0),
+    (8, 16, 16, (0.6, 0.3), 9), (4, 8, 16, (0.9,), 9),  # too little workspace to bin, chunks past a key per bucket
+])
+def test_segment_staged_inserts_where_binned_ones_would_do(cfb, orc, kb, bits, bs, loads, limit, results, dfs):
+    """The path that binned inserts fall back on: narrow entries, ranked claims in three
+    rounds, on an empty table and a filled one, with and without results."""
+    cfg = cfb.CuckooConfig(T="uint64" if kb == 8 else "uint32", bitsPerTag=bits, bucketSize=bs, maxEvictions=500,
+                           evictionPolicy=cfb.EvictionPolicy.DFS if dfs else cfb.EvictionPolicy.BFS)
+    f = cfb.CuckooFilter(cfg, 1 << 20)
+    if limit:
+        f.setOption(cfb.OPT_WORKSPACE_LIMIT, limit << 20)
+    else:
+        f.setOption(cfb.OPT_STAGING, cfb.STAGING_SEGMENT)
+    at, batches = 0, []
+    for load in loads:
+        n = int(load * f.capacity())
+        keys = orc.splitmix64(350 + bits + bs, n, first=at)
+        at += n
+        batches.append(dev(keys.astype(np.uint32) if kb == 4 else keys))
+    filled_and_emptied(cfb, f, batches, results, sorted_=True)
+    assert f.getOption(cfb.OPT_WORKSPACE_BYTES) <= (limit << 20 or 1 << 30)
+    f.close()
+
+
 @pytest.mark.parametrize("results,limit", [(False, 49 << 20), (True, 66 << 20)])
 @pytest.mark.parametrize("dfs", [False, True])
 def test_binned_insert_past_a_half_length_list(cfb, orc, results, limit, dfs):
