@@ -327,11 +327,6 @@ int staged_batch(cf_filter* f, void* stream, bool wait, uint64_t* occupied_out, 
     return st ? st : noted;
 }
 
-int ilog2(uint64_t v) { return 63 - __builtin_clzll(v); }
-
-// ceil(log2(v)) for v >= 1
-int clog2(uint64_t v) { return v <= 1 ? 0 : ilog2(v - 1) + 1; }
-
 void init_geometry(cf_filter* f) {
     const uint64_t bb = f->ops->bucket_bytes;
     uint64_t sb = kSegBytes / bb;
@@ -541,45 +536,6 @@ int run_segmented(cf_filter* f, int op, const void* keys, uint64_t n, uint8_t* o
     return CF_OK;
 }
 
-// Geometry of a binned insert of m keys (cf_binned.cuh), or false where the
-// path does not apply.  Segments are at most 64 KiB (three CTAs per SM), and
-// smaller in a small table, so that every SM gets one (2^20 slots: 256 segments
-// of 8 KiB take 6 us a round, 32 of 64 KiB took 45).
-bool bin_geometry(const cf_filter* f, uint64_t m, BinGeom* g) {
-    if (!f->ops->bin_insert || !f->seg_ok || m == 0 || m >= (1ull << 31)) return false;
-    const uint64_t nb = f->num_buckets, bb = f->ops->bucket_bytes;
-    if (nb > (1ull << 32)) return false;  // bucket indexes are 32-bit here
-    const int bits = static_cast<int>(f->cfg.bits_per_tag);
-    int sbl = ilog2(std::min<uint64_t>(kSegBytes / bb, nb));
-    while (sbl > 5 && ((nb - 1) >> sbl) + 1 < 256) --sbl;
-    const uint64_t nseg = ((nb - 1) >> sbl) + 1;
-    // two passes of equal fan-out past kBinMaxDigits segments
-    int l2 = nseg > kBinMaxDigits ? clog2(nseg) / 2 : 0;
-    if (l2 && bits < 32 && l2 + sbl + bits > 32 && sbl + bits < 32 && ((nseg - 1) >> (32 - bits - sbl)) + 1 <= kBinMaxDigits)
-        l2 = 32 - bits - sbl;  // unless some more first-pass bins keep the entries between the passes at 4 bytes
-    if ((1ull << l2) > kBinMaxDigits || ((nseg - 1) >> l2) + 1 > kBinMaxDigits) return false;
-    g->sbl = sbl;
-    g->l2 = l2;
-    g->nseg = static_cast<uint32_t>(nseg);
-    g->d1 = static_cast<uint32_t>(((nseg - 1) >> l2) + 1);
-    g->entry_bytes2 = bits < 32 ? 4 : 8;  // (at most 13 bits of bucket: 64 KiB of 8-byte buckets)
-    g->entry_bytes1 = g->entry_bytes2 == 4 && l2 + sbl + bits <= 32 ? 4 : 8;
-    // Room of a bin: the mean of evenly hashed keys plus six standard deviations
-    // (the AddSub policy's primary buckets are the first half of the table).
-    const double spread = static_cast<double>(f->cfg.alt_policy == CF_ALT_ADDSUB ? (nb + 1) / 2 : nb);
-    auto room = [&](int log2_buckets) {
-        const double mean = std::min(static_cast<double>(m), static_cast<double>(m) * std::ldexp(1.0, log2_buckets) / spread);
-        return (static_cast<uint64_t>(mean + 6.0 * std::sqrt(mean) + 64.0) + 7) / 8 * 8;
-    };
-    const uint64_t r2 = room(sbl), r1 = room(sbl + l2);
-    g->ent[0] = l2 ? g->d1 * r1 : nseg * r2;
-    g->ent[1] = nseg * r2;
-    if (g->ent[0] >= (1ull << 32) || g->ent[1] >= (1ull << 32)) return false;
-    g->room1 = static_cast<uint32_t>(r1);
-    g->room2 = static_cast<uint32_t>(r2);
-    return true;
-}
-
 // The whole batch through the binned path; *taken is false (and nothing has
 // been stored) when its workspace does not fit the limit or the batch is skewed.
 int run_binned(cf_filter* f, const void* keys, uint64_t n, uint8_t* out, void* stream, bool* taken) {
@@ -588,7 +544,9 @@ int run_binned(cf_filter* f, const void* keys, uint64_t n, uint8_t* out, void* s
     // workspace), so a capturing stream is left to the segment-staged path, whose
     // host waits end the capture with an error.
     BinGeom g{};
-    if (is_capturing(static_cast<cudaStream_t>(stream)) || !bin_geometry(f, n, &g)) return CF_OK;
+    if (is_capturing(static_cast<cudaStream_t>(stream)) || !f->ops->bin_insert || !f->seg_ok ||
+        !bin_geometry(f->num_buckets, f->ops->bucket_bytes, f->cfg.bits_per_tag, f->cfg.alt_policy, n, &g))
+        return CF_OK;
     auto al = [](uint64_t x) { return (x + 255) & ~255ull; };
     const uint64_t words = f->cfg.bucket_size <= 64 && g.sbl >= 5 ? (static_cast<uint64_t>(g.nseg) << g.sbl) >> 5 : 0;
     // a buffer holds first-pass bins in one round and segments' bins in another

@@ -20,6 +20,8 @@
 // is unspecified, in buckets of at most 16 slots; cf_segmented.cuh takes the rest.
 #pragma once
 
+#include <algorithm>
+#include <cmath>
 #include <cstdint>
 
 #include "cf_segmented.cuh"
@@ -49,6 +51,51 @@ struct BinGeom {
     int entry_bytes2;   // bytes of an entry of a segment's bin
     uint64_t ent[2];    // entries of the two bin buffers
 };
+
+inline int ilog2(uint64_t v) { return 63 - __builtin_clzll(v); }
+// ceil(log2(v)) for v >= 1
+inline int clog2(uint64_t v) { return v <= 1 ? 0 : ilog2(v - 1) + 1; }
+
+// Geometry of a binned insert of m keys into nb buckets of bb bytes, or false where
+// the path does not apply.  Segments are at most 64 KiB (three CTAs per SM), and
+// smaller in a small table, so that every SM gets one (2^20 slots: 256 segments
+// of 8 KiB take 6 us a round, 32 of 64 KiB took 45).
+inline bool bin_geometry(uint64_t nb, uint64_t bb, int bits, uint32_t alt_policy, uint64_t m, BinGeom* g) {
+    if (m == 0 || m >= (1ull << 31)) return false;
+    if (nb > (1ull << 32)) return false;  // bucket indexes are 32-bit here
+    int sbl = ilog2(std::min<uint64_t>(kSegBytes / bb, nb));
+    while (sbl > 5 && ((nb - 1) >> sbl) + 1 < 256) --sbl;
+    const uint64_t nseg = ((nb - 1) >> sbl) + 1;
+    // two passes of equal fan-out past kBinMaxDigits segments
+    int l2 = nseg > kBinMaxDigits ? clog2(nseg) / 2 : 0;
+    if (l2 && bits < 32 && l2 + sbl + bits > 32 && sbl + bits < 32 && ((nseg - 1) >> (32 - bits - sbl)) + 1 <= kBinMaxDigits)
+        l2 = 32 - bits - sbl;  // unless some more first-pass bins keep the entries between the passes at 4 bytes
+    if ((1ull << l2) > kBinMaxDigits || ((nseg - 1) >> l2) + 1 > kBinMaxDigits) return false;
+    g->sbl = sbl;
+    g->l2 = l2;
+    g->nseg = static_cast<uint32_t>(nseg);
+    g->d1 = static_cast<uint32_t>(((nseg - 1) >> l2) + 1);
+    g->entry_bytes2 = bits < 32 ? 4 : 8;  // (at most 13 bits of bucket: 64 KiB of 8-byte buckets)
+    g->entry_bytes1 = g->entry_bytes2 == 4 && l2 + sbl + bits <= 32 ? 4 : 8;
+    // Room of a bin: the mean of its keys plus six standard deviations.  The AddSub
+    // policy's primary buckets are the first half of the table.  Where a bucket is a
+    // 32-bit hash modulo a count that is no power of two, the first buckets get one
+    // hash value more than the last, which counts in large tables: 0.4 % of a bin's
+    // keys at 10^9 slots, against six deviations of 0.3 % (0.7 M keys had no room).
+    const uint64_t range = alt_policy == ALT_ADDSUB ? (nb + 1) / 2 : nb;
+    const uint64_t hashes = ((1ull << 32) + range - 1) / range;  // of a first bucket, of 2^32
+    auto room = [&](int log2_buckets) {
+        const double mean = std::min(static_cast<double>(m), static_cast<double>(m) * std::ldexp(static_cast<double>(hashes), log2_buckets - 32));
+        return (static_cast<uint64_t>(mean + 6.0 * std::sqrt(mean) + 64.0) + 7) / 8 * 8;
+    };
+    const uint64_t r2 = room(sbl), r1 = room(sbl + l2);
+    g->ent[0] = l2 ? g->d1 * r1 : nseg * r2;
+    g->ent[1] = nseg * r2;
+    if (g->ent[0] >= (1ull << 32) || g->ent[1] >= (1ull << 32)) return false;
+    g->room1 = static_cast<uint32_t>(r1);
+    g->room2 = static_cast<uint32_t>(r2);
+    return true;
+}
 
 // Device workspace of a binned batch.
 struct BinWork {
