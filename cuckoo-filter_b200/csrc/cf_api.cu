@@ -555,9 +555,11 @@ int run_binned(cf_filter* f, const void* keys, uint64_t n, uint8_t* out, void* s
     const uint64_t cursors = 3ull * ((g.l2 ? g.d1 : 0u) + g.nseg) * 4 * kCursorStride;
     // The list of entries without room holds the whole batch, or half of it (two
     // passes only) where the memory counts (8 GB at 2^30 keys) and the waits that
-    // go with it do not, or where only that fits the limit.  In a table that is not
-    // empty the first round can leave more than half of the batch, which a short list
-    // sends to random inserts, so there it has its full length if it can.
+    // go with it do not, or where only that fits the limit.  What the first round leaves
+    // goes to random inserts if a short list might not hold it (AddSub fill of 10^9 slots:
+    // 79 ms for 38), so the list has its full length, if it can, where that may be: in a
+    // table that is not empty, and where the primary buckets hold less than five
+    // eighths of the batch (the AddSub policy's are half of the table).
     // list, ent[0] and ent[1] side by side hold two lists of n entries in the end.
     uint64_t room = 0, ents = 0, pays = 0, need = 0;
     auto size = [&](uint64_t list_room) {
@@ -567,7 +569,10 @@ int run_binned(cf_filter* f, const void* keys, uint64_t n, uint8_t* out, void* s
         need = ents + pays + al(cursors) + al(g.nseg * 4ull) + al(64) + al(words * 4);
     };
     const bool can_halve = g.l2 && b0 >= n * 8 && (!out || g.ent[0] >= n);
-    size(can_halve && n >= (1ull << 27) && f->known_empty ? n / 2 : n);
+    const uint64_t bs = f->cfg.bucket_size, cap1 = f->round1_cap ? f->round1_cap : bs - bs * kRound1SlackSixteenths / 16;
+    const uint64_t primary = f->cfg.alt_policy == CF_ALT_ADDSUB ? f->num_buckets / 2 : f->num_buckets;
+    const bool leaves_few = f->known_empty && cap1 * primary >= n / 8 * 5;
+    size(can_halve && n >= (1ull << 27) && leaves_few ? n / 2 : n);
     if (need > f->ws_bytes) {
         const uint64_t limit = f->ws_limit ? f->ws_limit : auto_workspace_limit(f);
         if (need > limit && can_halve) size(n / 2);

@@ -280,6 +280,25 @@ def test_binned_insert_past_a_half_length_list(cfb, orc, results, limit, dfs):
     f.close()
 
 
+@pytest.mark.parametrize("alt,load,cap", [("xor", 0.6, 0), ("addsub", 0.95, 0), ("xor", 0.6, 2)])
+def test_large_binned_inserts_keep_their_rounds(cfb, alt, load, cap):
+    """Fills of 2^27 keys and more, where a list of half the batch would do and where the
+    first round leaves more than that: three rounds of binning all the same."""
+    cfg = cfb.CuckooConfig(T="uint64", bitsPerTag=16, bucketSize=16, AltBucketPolicy=POLICY[alt],
+                           evictionPolicy=cfb.EvictionPolicy.BFS)
+    f = cfb.CuckooFilter(cfg, int((1 << 27) / load) + (1 << 20) if alt != "xor" else 1 << 28)
+    if cap:
+        f.setOption(cfb.OPT_ROUND1_CAP, cap)
+    n = (1 << 27) + 12345
+    keys = torch.randint(-2 ** 63, 2 ** 63 - 1, (n,), device="cuda", generator=torch.Generator("cuda").manual_seed(9))
+    launches = launches_of(cfb, f, lambda: f.insertMany(keys))
+    assert launches >= 13, launches  # 3 x (2 binning passes, insert), then the lists
+    st = f.stats()
+    assert f.occupiedSlots() == f.countOccupiedSlots() == n and st["failed"] == st["lost"] == st["duplicates"] == 0
+    assert bool(f.containsMany(keys).all())
+    f.close()
+
+
 @pytest.mark.parametrize("bits,bs", [(8, 16), (16, 16), (32, 8)])
 @pytest.mark.parametrize("kpt", [1, 2, 4, 8])
 def test_set_items_that_end_inside_a_thread(cfb, orc, bits, bs, kpt):
