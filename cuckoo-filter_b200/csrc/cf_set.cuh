@@ -12,9 +12,9 @@
 //
 // Per-key semantics are the single-filter kernels' (cf_kernels.cuh): the
 // reference's insert / contains / remove (CuckooFilter.cuh:805-1116) applied
-// to the filter the key belongs to.  Counters are per filter; a warp whose keys
-// all belong to one filter (nearly every warp) adds each count with one
-// reduction and one atomic, any other with one atomic per distinct filter
+// to the filter the key belongs to.  Counters are per filter; each count is added
+// with one atomic per run of lanes whose keys belong to one filter (one prefix
+// scan finds the runs' sums), in the eviction with one per distinct filter
 // (__match_any_sync).
 //
 // Tunables (template parameters, picked by the set's autotuner): KPT keys per
@@ -37,13 +37,39 @@ __device__ __forceinline__ uint32_t set_find_item(const uint64_t* __restrict__ o
     return lo;
 }
 
+// The same over all items by the 32 lanes of a warp: four loads one after the other
+// for 10^5 items where the search above makes 17.
+__device__ __forceinline__ uint32_t set_find_item_warp(const uint64_t* __restrict__ offs, uint32_t n_items, uint64_t k) {
+    const uint32_t lane = threadIdx.x & 31;
+    uint32_t lo = 0, hi = n_items;
+    while (lo + 1 < hi) {
+        const uint32_t step = (hi - lo + 31) / 32;
+        const uint64_t at = lo + static_cast<uint64_t>(lane + 1) * step;
+        const uint32_t le = __ballot_sync(0xFFFFFFFFu, at < hi && offs[at] <= k);
+        const uint32_t c = static_cast<uint32_t>(__ffs(~le)) - 1u;  // (the last lane's is past hi)
+        const uint32_t end = hi - lo;
+        hi = (c + 1) * static_cast<uint64_t>(step) < end ? lo + (c + 1) * step : hi;
+        lo += c * step;
+    }
+    return lo;
+}
+
 // Items of the tile [first, last]: range[0] of its first key, range[1] past that
-// of its last.  Every thread of the CTA calls it, between two barriers of its own.
+// of its last (which is past range[0] whatever offs holds: both searches make the
+// same probes until the one for the later key goes further).  Every thread of the
+// CTA calls it, between two barriers of its own.
 __device__ __forceinline__ void set_tile_items(const uint64_t* __restrict__ offs, uint32_t n_items, uint64_t first,
                                                uint64_t last, uint32_t (&range)[2]) {
     __syncthreads();
-    if (threadIdx.x == 0) range[0] = set_find_item(offs, 0, n_items, first);
-    if (threadIdx.x == 32 % blockDim.x) range[1] = set_find_item(offs, 0, n_items, last) + 1;
+    const uint32_t warp = threadIdx.x / 32, lane = threadIdx.x & 31;
+    if (warp == 0) {
+        const uint32_t a = set_find_item_warp(offs, n_items, first);
+        if (lane == 0) range[0] = a;
+    }
+    if (warp == (blockDim.x > 32 ? 1u : 0u)) {
+        const uint32_t b = set_find_item_warp(offs, n_items, last) + 1;
+        if (lane == 0) range[1] = b;
+    }
     __syncthreads();
 }
 
@@ -94,6 +120,24 @@ __device__ __forceinline__ void set_add_ctrs(const DevTable* __restrict__ descs,
         }
         if (leader && s) atomicAdd(&descs[f].ctr[a[i].idx], static_cast<unsigned long long>(static_cast<long long>(s)));
     }
+}
+
+// Adds each lane's counts of its filter f, p and q (at most 32 each), where lanes of
+// one filter mostly lie side by side: one atomic per counter and run of such lanes,
+// add(ctr, sum of p, sum of q).  The runs' sums come from one prefix scan, so that
+// warps of many small items do no more than others.  All lanes of the warp must call it.
+template <class Add>
+__device__ __forceinline__ void set_add_runs(const DevTable* __restrict__ descs, uint32_t f, bool active, uint32_t p,
+                                             uint32_t q, Add add) {
+    const uint32_t lane = threadIdx.x & 31, act = __ballot_sync(0xFFFFFFFFu, active);
+    if (!act) return;
+    const uint32_t g = active ? f : 0xFFFFFFFFu, before = __shfl_up_sync(0xFFFFFFFFu, g, 1);
+    const uint32_t heads = __ballot_sync(0xFFFFFFFFu, lane == 0 || g != before);
+    const uint32_t incl = warp_inclusive_scan(active ? p << 16 | q : 0u);
+    const uint32_t prior = __shfl_up_sync(0xFFFFFFFFu, incl, 1);
+    const uint32_t next = lane < 31 ? heads & (0xFFFFFFFEu << lane) : 0u;  // heads past this lane
+    const uint32_t total = __shfl_sync(0xFFFFFFFFu, incl, next ? __ffs(next) - 2 : 31) - (lane ? prior : 0u);
+    if (active && ((heads >> lane) & 1u) && total) add(descs[f].ctr, total >> 16, total & 0xFFFFu);
 }
 
 // Keys of a thread that are probed together: their bucket loads overlap, and two
@@ -245,7 +289,10 @@ __global__ void __launch_bounds__(512) k_set_containsW(const DevTable* __restric
 // deleteMany over the set: each thread owns KPT consecutive keys.  The keys of
 // the thread's first filter are worked on together; those past the filter's end
 // (a few threads per item) follow one at a time, so the common path keeps one
-// table descriptor in registers.
+// table descriptor in registers.  Items of a few keys put several filters into a
+// thread: 1.3 M keys of 10^5 filters, four keys per thread, took 62 us with one
+// bucket load in flight, 110 with the warp's counts matched for every key past the
+// first filter, and take 65.
 template <class C, int KPT>
 __global__ void __launch_bounds__(512, 2) k_set_delete(const DevTable* __restrict__ descs, const uint32_t* __restrict__ filt,
                                                        const uint64_t* __restrict__ offs, uint32_t n_items,
@@ -298,34 +345,44 @@ __global__ void __launch_bounds__(512, 2) k_set_delete(const DevTable* __restric
                     try_remove<C>(bucket_words<C>(t, b[j]), c[j], alt_tag<C>(fp[j]), err))
                     gone |= 1u << (g + j);
         }
-        {
-            const int32_t r = __popc(gone);
-            set_add_ctrs(descs, f, live != 0, {{CTR_REMOVED, r}, {CTR_OCCUPIED, -r}});
-        }
-        for (uint32_t j = here; __any_sync(0xFFFFFFFFu, j < have); ++j) {  // keys past the first filter
-            bool ok = false, v = j < have;
-            if (v) {
-                walk.to(offs, n_items, k0 + j);
-                f = set_filter(filt, walk.item, n_filters);
-                bad |= f == n_filters;
-                v = f < n_filters;
-            }
-            if (v) {
-                const DevTable t2 = descs[f];
+        set_add_runs(descs, f, live != 0, __popc(gone), 0u, [](unsigned long long* ctr, uint32_t r, uint32_t) {
+            atomicAdd(&ctr[CTR_REMOVED], static_cast<unsigned long long>(r));
+            atomicAdd(&ctr[CTR_OCCUPIED], ~static_cast<unsigned long long>(r) + 1ull);
+        });
+        if (here < have) {  // keys past the first filter
+            uint32_t r = 0;
+            DevTable t2{};
+            auto flush = [&]() {
+                if (!r) return;
+                atomicAdd(&t2.ctr[CTR_REMOVED], static_cast<unsigned long long>(r));
+                atomicAdd(&t2.ctr[CTR_OCCUPIED], ~static_cast<unsigned long long>(r) + 1ull);
+                r = 0;
+            };
+            for (uint32_t j = here; j < have; ++j) {
+                if (walk.to(offs, n_items, k0 + j)) {
+                    flush();
+                    f = set_filter(filt, walk.item, n_filters);
+                    bad |= f == n_filters;
+                    if (f < n_filters) t2 = descs[f];
+                }
+                if (f == n_filters) continue;
                 uint64_t b;
                 uint32_t fp;
                 uint64_t c[C::nchunks];
                 candidates<C>(static_cast<uint64_t>(keys[k0 + j]), t2.nb_mask, b, fp);
                 load_rlx<C::bucket_bytes>(bucket_words<C>(t2, b), c);
-                ok = try_remove<C>(bucket_words<C>(t2, b), c, fp, err);
+                bool ok = try_remove<C>(bucket_words<C>(t2, b), c, fp, err);
                 if (!ok && !err) {
                     b = alt_bucket<C>(b, fp, t2.nb_mask);
                     load_rlx<C::bucket_bytes>(bucket_words<C>(t2, b), c);
                     ok = try_remove<C>(bucket_words<C>(t2, b), c, alt_tag<C>(fp), err);
                 }
-                gone |= (ok ? 1u : 0u) << j;
+                if (ok) {
+                    gone |= 1u << j;
+                    ++r;
+                }
             }
-            set_add_ctrs(descs, f, v, {{CTR_REMOVED, ok ? 1 : 0}, {CTR_OCCUPIED, ok ? -1 : 0}});
+            flush();
         }
         if (have && out) store_results<KPT>(out, k0, n, out_vec, gone);
     }
@@ -421,36 +478,43 @@ __global__ void __launch_bounds__(512, 2) k_set_insert(const DevTable* __restric
                     try_insert<C>(bucket_words<C>(t, b[j]), c[j], alt_tag<C>(fp[j]), err))
                     sec |= 1u << (g + j);
         }
-        {
-            const int32_t p = __popc(prim), q = __popc(sec);
-            set_add_ctrs(descs, f, live != 0, {{CTR_PRIMARY, p}, {CTR_SECONDARY, q}, {CTR_OCCUPIED, p + q}});
-        }
-        for (uint32_t j = here; __any_sync(0xFFFFFFFFu, j < have); ++j) {  // keys past the first filter
-            bool p = false, q = false, v = j < have;
-            if (v) {
-                walk.to(offs, n_items, k0 + j);
-                f = set_filter(filt, walk.item, n_filters);
-                bad |= f == n_filters;
-                v = f < n_filters;
-            }
-            if (v) {
-                const DevTable t2 = descs[f];
+        auto stored = [](unsigned long long* ctr, uint32_t p, uint32_t q) {
+            if (p) atomicAdd(&ctr[CTR_PRIMARY], static_cast<unsigned long long>(p));
+            if (q) atomicAdd(&ctr[CTR_SECONDARY], static_cast<unsigned long long>(q));
+            if (p + q) atomicAdd(&ctr[CTR_OCCUPIED], static_cast<unsigned long long>(p + q));
+        };
+        set_add_runs(descs, f, live != 0, __popc(prim), __popc(sec), stored);
+        if (here < have) {  // keys past the first filter
+            uint32_t p = 0, q = 0;
+            DevTable t2{};
+            for (uint32_t j = here; j < have; ++j) {
+                if (walk.to(offs, n_items, k0 + j)) {
+                    stored(t2.ctr, p, q);
+                    p = q = 0;
+                    f = set_filter(filt, walk.item, n_filters);
+                    bad |= f == n_filters;
+                    if (f < n_filters) t2 = descs[f];
+                }
+                if (f == n_filters) continue;
+                live |= 1u << j;
                 uint64_t b;
                 uint32_t fp;
                 uint64_t c[C::nchunks];
                 candidates<C>(static_cast<uint64_t>(keys[k0 + j]), t2.nb_mask, b, fp);
                 load_rlx<C::bucket_bytes>(bucket_words<C>(t2, b), c);
-                p = try_insert<C>(bucket_words<C>(t2, b), c, fp, err);
-                if (!p && !err) {
+                if (try_insert<C>(bucket_words<C>(t2, b), c, fp, err)) {
+                    prim |= 1u << j;
+                    ++p;
+                } else if (!err) {
                     b = alt_bucket<C>(b, fp, t2.nb_mask);
                     load_rlx<C::bucket_bytes>(bucket_words<C>(t2, b), c);
-                    q = try_insert<C>(bucket_words<C>(t2, b), c, alt_tag<C>(fp), err);
+                    if (try_insert<C>(bucket_words<C>(t2, b), c, alt_tag<C>(fp), err)) {
+                        sec |= 1u << j;
+                        ++q;
+                    }
                 }
-                live |= 1u << j;
-                prim |= (p ? 1u : 0u) << j;
-                sec |= (q ? 1u : 0u) << j;
             }
-            set_add_ctrs(descs, f, v, {{CTR_PRIMARY, p ? 1 : 0}, {CTR_SECONDARY, q ? 1 : 0}, {CTR_OCCUPIED, p || q ? 1 : 0}});
+            stored(t2.ctr, p, q);
         }
         if (have && out) store_results<KPT>(out, k0, n, out_vec, prim | sec);
         // park the keys whose buckets are both full

@@ -346,6 +346,44 @@ def test_set_items_that_end_inside_a_thread(cfb, orc, bits, bs, kpt):
     assert np.array_equal(res[:int((~half).sum())].cpu().numpy(), ok[~half].astype(np.uint8))
 
 
+@pytest.mark.parametrize("n_items", [1, 2, 31, 33, 1025, 40_000])
+@pytest.mark.parametrize("block,kpt", [(32, 1), (128, 8), (512, 4)])
+def test_set_of_many_small_items(cfb, orc, n_items, block, kpt):
+    """Items of 0 to 5 keys, many of them empty, a filter in several items: counters,
+    results and occupancy of every filter."""
+    cfg = cfb.CuckooConfig(T="uint64", bitsPerTag=16, bucketSize=16, evictionPolicy=cfb.EvictionPolicy.BFS)
+    nf = max(1, n_items // 2)
+    fs = cfb.CuckooFilterSet(cfg, [64] * nf)
+    rng = np.random.default_rng(n_items + kpt)
+    sizes = rng.choice([0, 0, 1, 2, 3, 5], n_items)
+    sizes[-1] = 4
+    filt = rng.permutation(n_items).astype(np.int32) % nf  # at most 3 items, 15 keys, per filter
+    offs = np.concatenate([[0], np.cumsum(sizes)]).astype(np.int64)
+    keys, owner = orc.splitmix64(401, int(offs[-1])), np.repeat(filt, sizes)
+    for op in (cfb.SET_INSERT, cfb.SET_CONTAINS, cfb.SET_DELETE):
+        fs.set_launch(op, block, kpt)
+    d, o, w = dev(keys), torch.from_numpy(offs).cuda(), torch.from_numpy(filt).cuda()
+    res = torch.full((len(keys),), 7, dtype=torch.uint8, device="cuda")
+    want = np.bincount(owner, minlength=nf)
+    fs.insert_async(d, o, w, res)
+    fs.sync()
+    assert bool((res == 1).all()) and np.array_equal(fs.occupied(), want)
+    for i in rng.integers(0, nf, 50):
+        st = fs.stats(int(i))
+        assert st["primary"] + st["secondary"] == want[i] and st["evicted_inserts"] == 0
+    fs.contains_async(d, o, w, res.fill_(7))
+    fs.sync()
+    assert bool((res == 1).all())
+    fs.delete_async(d, o, w, res.fill_(7))
+    fs.sync()
+    assert bool((res == 1).all()) and int(fs.occupied().sum()) == 0
+    for i in rng.integers(0, nf, 50):
+        assert fs.stats(int(i))["removed"] == want[i]
+    fs.delete_async(d, o, w, res)
+    fs.sync()
+    assert int(res.sum()) == 0 and int(fs.occupied().sum()) == 0
+
+
 @pytest.mark.parametrize("kb,bits,bs,load", [(8, 16, 16, 0.99), (4, 8, 16, 0.98), (8, 8, 8, 0.95), (8, 32, 8, 0.97),
                                              (8, 16, 4, 0.93), (8, 32, 2, 0.86)])
 def test_short_eviction_lists(cfb, orc, kb, bits, bs, load):
