@@ -315,6 +315,9 @@ __device__ bool try_remove(uint64_t* bw, uint64_t (&c)[C::nchunks], uint32_t fp,
 // when some slot equals fp) and tested for a zero lane once per bucket, 32-bit
 // lanes are compared one by one, 8-bit lanes are tested for a zero lane word by
 // word (the borrow form: exact as a yes/no answer).
+// Buckets of 256 bytes keep 64-bit lane flags: the fold is one chain through all 64
+// words, and 4 M stored keys in 256 MiB took 225 us with it, 191 without (absent keys
+// 468 and 419; in 8 MiB the same); buckets of 128 bytes 121 with it, 128 without.
 template <class C>
 __device__ __forceinline__ bool has_tag(const uint64_t (&c)[C::nchunks], uint32_t fp) {
     if constexpr (C::bits == 32) {
@@ -323,6 +326,12 @@ __device__ __forceinline__ bool has_tag(const uint64_t (&c)[C::nchunks], uint32_
         for (int j = 0; j < C::nchunks; ++j)
             any = any || static_cast<uint32_t>(c[j]) == fp || static_cast<uint32_t>(c[j] >> 32) == fp;
         return any;
+    } else if constexpr (C::bits == 16 && C::nchunks > 16) {
+        const uint64_t rep = replicate<C::bits>(fp);
+        uint64_t any = 0;
+#pragma unroll
+        for (int j = 0; j < C::nchunks; ++j) any |= zero_lanes<C::bits>(c[j] ^ rep);
+        return any != 0;
     } else if constexpr (C::bits == 16) {
         const uint32_t rep = fp * 0x00010001u;
         uint32_t m = 0xFFFFFFFFu;
