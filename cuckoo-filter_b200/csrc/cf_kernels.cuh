@@ -22,7 +22,7 @@
 //     negative);
 //   * every compare-and-swap retry loop is bounded; hitting the bound sets an
 //     error flag that the host turns into a status code;
-//   * counters are accumulated per thread and flushed once per warp.
+//   * counters are accumulated per thread and added once per CTA.
 #pragma once
 
 #include <cstdint>
@@ -580,7 +580,7 @@ struct CounterAdd {
 // (up to 512 each) do not fit fewer.
 template <int N>
 __device__ __forceinline__ void flush_counters(unsigned long long* ctr, const CounterAdd (&a)[N]) {
-    static_assert(N <= 32, "lane i adds counter i");
+    static_assert(N <= 8, "lanes i, 8 + i, 16 + i and 24 + i add counter i");
     __shared__ long long s_part[32][N];
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = (blockDim.x + 31) >> 5;
 #pragma unroll
@@ -591,14 +591,15 @@ __device__ __forceinline__ void flush_counters(unsigned long long* ctr, const Co
     }
     __syncthreads();
     if (warp != 0) return;
-    if (lane < N) {
-        int idx = 0;
-        long long s = 0;
+    int idx = 0;
+    long long s = 0;
 #pragma unroll
-        for (int i = 0; i < N; ++i) idx = static_cast<int>(lane) == i ? a[i].idx : idx;
-        for (uint32_t w = 0; w < nwarp; ++w) s += s_part[w][lane];
-        if (s) atomicAdd(&ctr[idx], static_cast<unsigned long long>(s));
-    }
+    for (int i = 0; i < N; ++i) idx = static_cast<int>(lane) == i ? a[i].idx : idx;
+    if ((lane & 7) < N)
+        for (uint32_t w = lane >> 3; w < nwarp; w += 4) s += s_part[w][lane & 7];
+    s += __shfl_down_sync(0xFFFFFFFFu, s, 16);
+    s += __shfl_down_sync(0xFFFFFFFFu, s, 8);
+    if (lane < N && s) atomicAdd(&ctr[idx], static_cast<unsigned long long>(s));
     __syncwarp();
 }
 
