@@ -678,22 +678,23 @@ def run_b200(args, w: dict) -> dict | None:
            "contains": {**op(n_q, con_ms, con_bytes), "ms_steps": con_ms},
            "delete": {**op(n_d, del_ms, del_bytes), "ms_steps": del_ms}, "clear_ms": statistics.mean(
                [evs[k][0].elapsed_time(evs[k][1]) for k in range(args.steps)])}
-    # the library's automatic choice (CF_OPT_SEGMENTED_MIN_KEYS = 0): inserts are
-    # segment-staged from one key per bucket, lookups and deletes from eight
-    def path_of(n, per_bucket):
-        if args.staging != "auto":
-            return {"random": "random probes", "segment": "segment-staged", "region": "region-staged"}[args.staging]
-        return "segment-staged" if n >= f.getNumBuckets() * per_bucket else "random probes"
-
-    ins_path = path_of(n_fill, 1)
-    ops["insert"]["path"] = ("insertManySorted (segment-staged)" if sorted_fill and args.staging != "region" else
-                             "insertManySorted (region-staged)" if sorted_fill else
-                             "insertMany (random CAS)" if ins_path == "random probes" else f"insertMany ({ins_path})")
-    ops["contains"]["path"] = path_of(n_q, 8)
-    ops["delete"]["path"] = path_of(n_d, 8)
+    # the library's automatic choice (CF_OPT_SEGMENTED_MIN_KEYS = 0): inserts of one key per
+    # bucket and 2^17 keys (2^20 below three quarters load) on are staged, binned where buckets
+    # have at most 16 slots; lookups probe at random, deletes below eight keys per bucket
+    forced = {"auto": None, "random": "random probes", "segment": "segment-staged", "region": "region-staged"}[args.staging]
+    nb = f.getNumBuckets()
+    staged = "binned" if n_fill >= nb and w["bs"] <= 16 and args.staging != "segment" else "segment-staged"
+    least = max(nb, 1 << 17 if n_fill >= 0.75 * f.capacity() else 1 << 20)
+    if sorted_fill:
+        ops["insert"]["path"] = f"insertManySorted ({'region-staged' if args.staging == 'region' else staged})"
+    else:
+        ins_path = forced or (staged if n_fill >= least else "random probes")
+        ops["insert"]["path"] = "insertMany (random CAS)" if ins_path == "random probes" else f"insertMany ({ins_path})"
+    ops["contains"]["path"] = forced or "random probes"
+    ops["delete"]["path"] = forced or ("segment-staged" if n_d >= 8 * nb else "random probes")
 
     # plain insertMany on the random CAS path (a fill this large would be
-    # segment-staged by default), on the same fill, timed on its own
+    # binned by default), on the same fill, timed on its own
     if sorted_fill and not args.no_plain:
         f.setOption(cfb.OPT_STAGING, cfb.STAGING_RANDOM)
         ts = []
@@ -858,7 +859,7 @@ def verify_parity(f, w: dict, fill, query, is_pos, dele, sorted_fill: bool, stre
     """Per-key parity of the timed configuration on the full workload (untimed).
 
     The fill is the timed steps' own (library defaults: for a large batch the
-    capped three-round segment-staged insert).  Then:
+    capped three-round staged insert).  Then:
       * counters against the image: occupied == countOccupiedSlots == stored
         keys, lost == 0;
       * zero false negatives over every stored fill key;
@@ -1375,7 +1376,7 @@ def _time_fill_query_delete(cfb, f, path, fill, query, dele, q_out, stream) -> d
     f.clear(stream)
     f.resetEvictionCount()
     e = [torch.cuda.Event(enable_timing=True) for _ in range(4)]
-    # a fill this large would be segment-staged by default: force random CAS
+    # a fill this large would be binned by default: force random CAS
     f.setOption(cfb.OPT_STAGING, cfb.STAGING_RANDOM if path == "insertMany" else cfb.STAGING_AUTO)
     e[0].record(stream)
     if path == "insertMany":
@@ -1995,7 +1996,7 @@ def main() -> None:
                     help="fill with insertMany (plain), insertManySorted (sorted), or as the reference's benchmark "
                          "does (auto: sorted from 2^29 keys)")
     ap.add_argument("--workspace-gb", type=float, default=None,
-                    help="workspace limit of the segment-staged path (CF_OPT_WORKSPACE_LIMIT); default: the "
+                    help="workspace limit of the staged paths (CF_OPT_WORKSPACE_LIMIT); default: the "
                          "library's own (automatic) limit")
     ap.add_argument("--no-forms", action="store_true",
                     help="skip the brief batched / served forms in the default line")

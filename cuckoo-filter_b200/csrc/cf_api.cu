@@ -477,15 +477,11 @@ int ensure_workspace(cf_filter* f, uint64_t n, bool payload, SegWork* w) {
     return CF_OK;
 }
 
-// Keys from which the segment-staged path beats random probes: a random probe
-// costs one DRAM transaction, streaming a segment costs its bytes (read, and
-// write-back for insert/delete).
-// Measured on B200: a random probe costs one DRAM transaction (the device
-// completes ~38 G/s); the segment path costs its radix passes, the streamed
-// segments and the shared-memory work.  Lookups and deletes beat random
-// probing on the segment path only for batches of several keys per bucket;
-// the alternate-bucket round of a segment batch pays off from about one key
-// per 64 table bytes.
+// Keys from which the alternate-bucket round of a segment-staged batch is staged too
+// rather than probed at random: a random probe costs one DRAM transaction (about
+// 50 G/s for reads of a table past L2, 23 for read-modify-writes), staging the segments'
+// bytes, read and for inserts written back.  For inserts that pays off from about
+// one key per 64 table bytes, for lookups and deletes from several keys per bucket.
 uint64_t auto_threshold(const cf_filter* f, int op) {
     if (op == SEG_INSERT) return f->table_bytes / 64;
     return f->num_buckets * 8;
@@ -493,10 +489,14 @@ uint64_t auto_threshold(const cf_filter* f, int op) {
 
 // Batch size from which a batch is staged.  Inserts: one key per bucket, and
 // enough keys to pay for a dozen launches: 2^17, or 2^20 for batches that cannot
-// fill the table beyond three quarters (fewer evictions, which random inserts
-// pay most for).  Binned against random, us, 16-bit tags, filling an empty table:
+// fill an empty table beyond three quarters (fewer evictions, which random inserts
+// pay most for; the load before the batch is not known on the host, and tops-up
+// from 0.6 and 0.8 to 0.9 were faster at random than segment-staged too).  Binned against random, us, 16-bit tags, filling an empty table:
 // 2^14 slots to 0.95 80 and 58, to 0.6 52 and 25; 2^17 to 0.6 60 and 28; 2^20 to 0.6
 // 66 and 40, to 0.95 107 and 110; 2^22 to 0.6 80 and 92, to 0.95 156 and 236.
+// (Batches full of repeats are the exception: keys that must fail walk to the end
+// beside the others.  2^18 slots to 0.6, half the batch repeats of 100 keys, DFS: 4.3 ms
+// at random, 3.0 segment-staged.)
 // Below one key per bucket random inserts win at every size (2^26 8-bit slots,
 // 0.76 keys per bucket: 105 us a batch in the first half of the fill, 170 in the
 // second, against 309 and 382 segment-staged).
@@ -625,7 +625,7 @@ int run_binned(cf_filter* f, const void* keys, uint64_t n, uint8_t* out, void* s
 }
 
 // Region-staged path (cf_region.cuh): keys from which it beats random probes.
-// A random probe costs one DRAM transaction (~38 G/s on B200); the region path
+// A random probe costs one DRAM transaction (~50 G/s on B200); the region path
 // streams ~30 bytes per key plus the table once (lookups) or about twice
 // (inserts and deletes), at close to HBM bandwidth.
 uint64_t region_threshold(const cf_filter* f, int op) {

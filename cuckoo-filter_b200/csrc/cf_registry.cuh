@@ -74,7 +74,11 @@ constexpr int kRgGatherMaxSmem = 160 * 1024;
 // share of the list; more, smaller shares were measured faster on B200).
 constexpr int kEvictGridWaves = 4;
 // Batch size up to which a binned insert evicts with NC lanes per key (see
-// k_evict_bfs_coop; the lockstep pass overtook it between 32 M and 64 M keys).
+// k_evict_bfs_coop; the lockstep pass overtook it between 32 M and 64 M keys).  The
+// host does not know the list's length, which follows the batch's for keys that
+// hash evenly; the long list of a smaller batch full of repeats would be better off
+// with the lockstep pass (2^25 slots to 0.6, half the batch repeats of 10^4 keys:
+// 210 ms, 140 with it).
 constexpr uint64_t kCoopEvictBatch = 1ull << 25;
 // Slots of each bucket (in sixteenths) that the first round of a large
 // segment-staged insert leaves free for the second round.
