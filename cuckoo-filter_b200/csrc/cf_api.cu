@@ -276,13 +276,13 @@ bool is_capturing(cudaStream_t s) {
 int follow_staged_locked(cf_filter* f, void* stream) {
     if (!f->staged_pending) return CF_OK;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
+    if (is_capturing(s)) return CF_OK;
     unsigned long long id = 0;  // of the stream itself: a handle can be used again for another
     if (cudaStreamGetId(s, &id) == cudaSuccess) {
         if (id == f->staged_stream) return CF_OK;
     } else {
         cudaGetLastError();
     }
-    if (is_capturing(s)) return CF_OK;
     CF_CUDA(cudaStreamWaitEvent(s, f->staged_ev, 0), "wait for the batch before");
     return CF_OK;
 }

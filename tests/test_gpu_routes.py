@@ -588,6 +588,36 @@ def test_staged_batches_on_two_streams(cfb, orc, staging, results):
     f.close()
 
 
+def test_capture_beside_an_asynchronous_staged_batch(cfb, orc):
+    """Random calls are captured and replayed on one stream although the last staged
+    batch, on another, has only been waited for by the caller."""
+    cfg = cfb.CuckooConfig(T="uint64", bitsPerTag=16, bucketSize=16, evictionPolicy=cfb.EvictionPolicy.BFS)
+    f = cfb.CuckooFilter(cfg, 1 << 22)
+    many, few = dev(orc.splitmix64(361, 2 << 20)), dev(orc.splitmix64(362, 1000))
+    found, gone = (torch.zeros(1000, dtype=torch.bool, device="cuda") for _ in range(2))
+    s1, s2 = torch.cuda.Stream(), torch.cuda.Stream()
+    f.insertMany(few), f.containsMany(few, found), f.deleteMany(few, gone)  # modules loaded
+    torch.cuda.synchronize()
+    f.insertManyAsync(many, stream=s1)
+    torch.cuda.synchronize()
+    found.zero_(), gone.zero_()
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, stream=s2):
+        f.insertManyAsync(few, stream=s2)
+        f.containsManyAsync(few, found, stream=s2)
+        f.deleteManyAsync(few, gone, stream=s2)
+    assert f.occupiedSlots() == many.numel()  # nothing has run yet
+    for _ in range(2):
+        g.replay()
+        torch.cuda.synchronize()
+        assert bool(found.all()) and bool(gone.all())
+        assert f.occupiedSlots() == f.countOccupiedSlots() == many.numel()
+        found.zero_(), gone.zero_()
+    assert bool(f.containsMany(many).all())
+    f.close()
+
+
 def test_counters_read_after_an_asynchronous_staged_batch(cfb, orc):
     """Every read of the counters waits for the staged batch before it, on a stream
     that the legacy default stream does not wait for by itself."""
